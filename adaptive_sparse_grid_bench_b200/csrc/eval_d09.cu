@@ -1,7 +1,11 @@
-/* Evaluation kernels for d = 9 (see eval_impl.cuh); one dimension per file
- * so the instantiations compile in parallel. */
+/* Evaluation kernels for d = 9 (see eval_impl.cuh); one dimension per file and
+ * one kernel per SG_EVAL_PART so that they compile in parallel. */
 #include "eval_impl.cuh"
 
-template int eval_launch<9>(const EvalArgs &, int, int, void *);
-template int eval_setup<9>();
-template int eval_batch_launch<9>(const EvalArgs *, const int2 *, int, int, int, void *);
+#if SG_EVAL_PART == 0
+template int eval_launch<9>(const EvalArgs *, void *);
+#elif SG_EVAL_PART == 1
+template int eval_batch_launch<9>(const EvalArgs *, const int2 *, int, void *);
+#else
+template int eval_shared_launch<9>(const EvalArgs *, const int2 *, int, const EvalArgs *, void *);
+#endif

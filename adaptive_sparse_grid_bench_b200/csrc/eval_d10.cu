@@ -1,7 +1,11 @@
-/* Evaluation kernels for d = 10 (see eval_impl.cuh); one dimension per file
- * so the instantiations compile in parallel. */
+/* Evaluation kernels for d = 10 (see eval_impl.cuh); one dimension per file and
+ * one kernel per SG_EVAL_PART so that they compile in parallel. */
 #include "eval_impl.cuh"
 
-template int eval_launch<10>(const EvalArgs &, int, int, void *);
-template int eval_setup<10>();
-template int eval_batch_launch<10>(const EvalArgs *, const int2 *, int, int, int, void *);
+#if SG_EVAL_PART == 0
+template int eval_launch<10>(const EvalArgs *, void *);
+#elif SG_EVAL_PART == 1
+template int eval_batch_launch<10>(const EvalArgs *, const int2 *, int, void *);
+#else
+template int eval_shared_launch<10>(const EvalArgs *, const int2 *, int, const EvalArgs *, void *);
+#endif

@@ -14,21 +14,23 @@
  * shared by all subspaces below a node.  Below a prefix cell the walk reads
  * one block: every subspace of the three innermost dims (C = d-3, A = d-2,
  * B = d-1), stored contiguously in the block layout (sg_layout.h) with dim
- * B's levels as paths: per finest cell t_L of a row, the L+1 surpluses a
- * point in that cell needs, side by side.  The surplus of (c, a, b) sits at
- *     base + coff(c) + t_c sub(R-c) + aoff(a) + t_a plen(a) + t_L (L+1) + b:
+ * B's levels of a row (c, a) folded into what a point needs of them: one
+ * surplus (L = 0), a pair of surpluses (L = 1), or the value and slope of the
+ * levels' piecewise linear sum on the point's half cell (L >= 2), at
+ *     base + coff(c) + t_c sub(R-c) + aoff(a) + t_a plen(a) + 2 t_B:
  *   - blocks follow each other in walk order, so the block base is a running
  *     counter plus one multiply-add per point (no table);
- *   - a row's L+1 loads share one address (the point's path) and differ by
- *     a constant, so each subspace costs one gather and one FMA, the row one
- *     address; the hats of dim B are precomputed per point in registers,
- *     those of dims A and C in this thread's column of shared memory;
+ *   - a row of L+1 subspaces costs one address, one load (4 or 8 bytes) and
+ *     one or two FMAs; the hats of dim B's levels 0 and 1 and the positions in
+ *     the halves of levels 2..kYReg+1 are precomputed per point in registers
+ *     (deeper rows, 10 % of the rows at d = 10, n = 10, compute theirs), the
+ *     hats of dims A and C in this thread's column of shared memory;
  *   - the two points of a thread are computed with Blackwell's packed FP32x2
  *     instructions (FFMA2, FADD2, FMUL2 through __ffma2_rn, __fadd2_rn,
  *     __fmul2_rn): one instruction does both points' FMA, product or
  *     compensated add, with each point's rounding exactly as in scalar code,
  *     so results are bit-identical to one point per thread;
- *   - blocks of budget R <= kRFof<BL> run fully unrolled; larger blocks
+ *   - blocks of budget R <= kRFof<D> run fully unrolled; larger blocks
  *     loop over their planes and run each plane's 2-D sub-block fully
  *     unrolled behind a jump table.  A block or sub-block whose budget is within the limits of
  *     its dims has the regular shape whatever the limits, so limit-vector
@@ -37,14 +39,9 @@
  *   - most blocks sit under walk nodes of small remaining budget (at d=10,
  *     n=10, 8,008 of 11,440 blocks hold at most 4 subspaces), where loop and
  *     dispatch cost more than the gathers: the last prefix dim with budget
- *     <= kLGof<P, BL> (levels and blocks) and the last two with budget
+ *     <= SG_EVAL_MAX_LEAF (levels and blocks) and the last two with budget
  *     <= kLG2 run as fully unrolled code with compile-time block sizes, in
  *     walk order, so results are bit-identical to the loop (d <= kMaxUnrollD);
- *   - BL is the subspace blocking preset, a template parameter (wide = 0,
- *     medium = 1; the autotuner picks one per grid or per dimension of a
- *     batch): more unrolled code saves loop and dispatch work but raises
- *     register pressure, and the best trade depends on the grid and on the
- *     kernel (the batched kernel holds more state);
  *   - per prefix dim the walk keeps three values per point: the fractional
  *     part y = frac(x 2^l) (next level: doubling, exact in FP32), the cell
  *     index of the prefix (next level: 2*ix + bit) and the parent's product;
@@ -68,10 +65,12 @@ constexpr int kThreads = 256;
 constexpr int kNB = 10; /* 2-D sub-blocks of budget r < kNB run fully unrolled */
 constexpr int kRF = SG_EVAL_MAX_RF; /* 3-D blocks of budget R <= kRF can run unrolled */
 static_assert(kRF == 6, "block_sum's jump table covers budgets 0..6");
-/* largest budget of an unrolled 3-D block under blocking preset BL */
-template <int BL>
-constexpr int kRFof = BL == 0 ? kRF : 5;
+/* largest budget of an unrolled 3-D block (above 12 dims, where the walk's own
+ * state is larger, blocks of budget 6 only add spills) */
+template <int D>
+constexpr int kRFof = D <= 12 ? kRF : 5;
 constexpr int kTB = 15; /* T = floor(x 2^15) holds the cells of levels 0..15   */
+constexpr int kYReg = 1; /* positions in the halves of levels 2..kYReg+1 sit in registers */
 
 /* P floats of one thread's points: float2 (packed FP32x2 instructions) for
  * P = 2, a plain float for P = 1. */
@@ -145,21 +144,63 @@ __device__ __forceinline__ FV<P> hats(const FV<P> &y)
     return h;
 }
 
+/* The walk's view of arguments that sit in shared memory: the scalars it
+ * uses everywhere in registers, the tables read in place. */
+struct GridView {
+    const float *alpha;
+    int nm1, lim2, lim3;
+    const int *lim;
+    const uint32_t *blk3, *blk2, *seg;
+    __device__ __forceinline__ explicit GridView(const EvalArgs &A)
+        : alpha(A.alpha), nm1(A.nm1), lim2(A.lim2), lim3(A.lim3), lim(A.lim), blk3(A.blk3), blk2(A.blk2), seg(A.seg)
+    {
+    }
+};
+
+/* A hat from this thread's column of shared memory.  Written as assembly so
+ * that the compiler does not look for the thousands of possibly equal loads of
+ * the unrolled blocks (which took minutes per kernel) nor keeps their values in
+ * registers across blocks; a block reads each hat it needs once.  The columns
+ * are written once, before a compiler barrier, and only read after it. */
+template <int P>
+__device__ __forceinline__ FV<P> lds_hat(uint32_t column, int slot)
+{
+    static_assert(P == 2, "two points per thread");
+    FV<P> h;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                 : "=f"(h.v.x), "=f"(h.v.y)
+                 : "r"(column + (uint32_t)slot * (uint32_t)(kThreads * sizeof(FV<P>))));
+    return h;
+}
+
 /* Per-point values of the three innermost dims. */
 template <int P>
 struct Inner {
-    FV<P> hB[kNB];        /* hat of dim B at level b                 */
-    uint32_t TB[P];       /* floor(x_B 2^15): the path t_L = TB >> (15 - L) */
-    const FV<P> *sh;      /* this thread's hats of dims A, C in smem */
+    FV<P> hB[2];          /* hat of dim B at levels 0, 1             */
+    FV<P> yB[kYReg > 0 ? kYReg : 1]; /* frac(x_B 2^(L+1)), L = 2 ..       */
+    FV<P> xB;
+    uint32_t TB[P];       /* floor(x_B 2^15): cells and halves of dim B */
+    uint32_t sh;          /* shared address of this thread's hats of dims A, C */
     uint32_t TA[P];       /* floor(x_A 2^15): t_a = TA >> (15 - a)   */
     uint32_t TC[P];       /* floor(x_C 2^15)                         */
-    __device__ __forceinline__ FV<P> hA(int a) const { return sh[a * kThreads]; }
-    __device__ __forceinline__ FV<P> hC(int c) const { return sh[(kNB + c) * kThreads]; }
+    __device__ __forceinline__ FV<P> hA(int a) const { return lds_hat<P>(sh, a); }
+    /* position in the half of a cell of level L >= 2: frac(x_B 2^(L+1)),
+     * exact (the scaling and the difference are) */
+    __device__ __forceinline__ FV<P> y(int L) const
+    {
+        if (L - 2 < kYReg) return yB[L - 2];
+        const FV<P> t = vmul(xB, FV<P>::all((float)(2u << L)));
+        FV<P> f;
+#pragma unroll
+        for (int p = 0; p < P; ++p) f.set(p, truncf(t.get(p)));
+        return vsub(t, f);
+    }
+    __device__ __forceinline__ FV<P> hC(int c) const { return lds_hat<P>(sh, kNB + c); }
 };
 constexpr int kHatSlots = kNB + kRF + 1;
 
 /* Regular shapes: blocks whose budget is within the innermost limits. */
-__host__ __device__ constexpr uint32_t plen_reg(int r, int a) { return (1u << (r - a)) * (uint32_t)SG_PATH_WIDTH(r - a + 1); }
+__host__ __device__ constexpr uint32_t plen_reg(int r, int a) { return SG_POLE_SLOTS(r - a); }
 __host__ __device__ constexpr uint32_t aoff_reg(int r, int a)
 {
     uint32_t o = 0;
@@ -174,58 +215,134 @@ __host__ __device__ constexpr uint32_t coff_reg(int R, int c)
     return o;
 }
 
-/* 2-D sub-block of budget r: rows a = 0..r, row a holds 2^a poles of r-a+1
- * levels.  Returns sum_a hA[a] sum_b hB[b] alpha[...]. */
-template <int r, int P>
-__device__ __forceinline__ void block2_fixed(const float *__restrict__ alpha, const uint32_t (&base)[P],
-                                             const Inner<P> &in, FV<P> &s)
+/* A row of dim B with last level L, in two parts so that a block's loads can
+ * all be in flight before its first sum: what the point needs of the row at
+ * `at` (one load, sg_layout.h), and from it the sum over the row's levels of
+ * surplus * hat. */
+template <int P>
+struct RowData {
+    float2 w[P]; /* L = 0: .x only */
+};
+template <int L, int P>
+__device__ __forceinline__ void row_load(const float *__restrict__ alpha, const uint32_t (&at)[P], const Inner<P> &in,
+                                         RowData<P> &d)
 {
 #pragma unroll
-    for (int a = 0; a <= r; ++a) {
-        const int L = r - a; /* compile-time after unrolling */
-        const float *path[P]; /* the point's path: its L+1 surpluses of this row */
-#pragma unroll
-        for (int p = 0; p < P; ++p)
-            path[p] = alpha + (base[p] + aoff_reg(r, a) + cell_at(in.TA[p], a) * plen_reg(r, a) +
-                               cell_at(in.TB[p], L) * (uint32_t)SG_PATH_WIDTH(L + 1));
-        FV<P> sr = FV<P>::all(0.0f);
-        /* slots 2j, 2j+1 in one 8-byte load (paths of L >= 1 start even) */
-#pragma unroll
-        for (int b = 0; b + 1 <= L; b += 2) {
-            float2 w[P];
-#pragma unroll
-            for (int p = 0; p < P; ++p) w[p] = __ldg(reinterpret_cast<const float2 *>(path[p] + b));
-            FV<P> v0, v1;
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                v0.set(p, w[p].x);
-                v1.set(p, w[p].y);
-            }
-            sr = vfma(in.hB[b], v0, sr);
-            sr = vfma(in.hB[b + 1], v1, sr);
-        }
-        if ((L & 1) == 0) {
-            FV<P> v;
-#pragma unroll
-            for (int p = 0; p < P; ++p) v.set(p, __ldg(path[p] + L));
-            sr = vfma(in.hB[L], v, sr);
-        }
-        s = (a == 0) ? vmul(in.hA(0), sr) : vfma(in.hA(a), sr, s);
+    for (int p = 0; p < P; ++p) {
+        if constexpr (L == 0)
+            d.w[p].x = __ldg(alpha + at[p]);
+        else
+            d.w[p] = __ldg(reinterpret_cast<const float2 *>(
+                alpha + (at[p] + 2 * cell_at(in.TB[p], L == 1 ? 1 : L + 1))));
     }
+}
+template <int L, int P>
+__device__ __forceinline__ FV<P> row_sum(const RowData<P> &d, const Inner<P> &in)
+{
+    FV<P> v0, v1;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        v0.set(p, d.w[p].x);
+        if constexpr (L > 0) v1.set(p, d.w[p].y);
+    }
+    if constexpr (L == 0) return vmul(in.hB[0], v0);
+    else if constexpr (L == 1) return vfma(in.hB[1], v1, vmul(in.hB[0], v0));
+    else return vfma(in.y(L), v1, v0);
+}
+
+/* address of this point's pole in row a of a sub-block of budget r */
+template <int r, int a, int P>
+__device__ __forceinline__ void row_at(const uint32_t (&base)[P], const Inner<P> &in, uint32_t (&at)[P])
+{
+#pragma unroll
+    for (int p = 0; p < P; ++p) at[p] = base[p] + aoff_reg(r, a) + cell_at(in.TA[p], a) * plen_reg(r, a);
+}
+/* address of this point's sub-block in plane c of a block of budget R */
+template <int R, int c, int P>
+__device__ __forceinline__ void plane_at(const uint32_t (&base)[P], const Inner<P> &in, uint32_t (&sb)[P])
+{
+#pragma unroll
+    for (int p = 0; p < P; ++p) sb[p] = base[p] + coff_reg(R, c) + cell_at(in.TC[p], c) * blk2_reg(R - c);
+}
+
+/* 2-D sub-block of budget r: rows a = 0..r, row a holds 2^a poles of r-a+1
+ * levels.  s = sum_a hA[a] * (row sum). */
+template <int r, int a, int P, int NA>
+__device__ __forceinline__ void block2_fixed(const float *__restrict__ alpha, const uint32_t (&base)[P],
+                                             const Inner<P> &in, const FV<P> (&hA)[NA], FV<P> &s)
+{
+    uint32_t at[P];
+    RowData<P> d;
+    row_at<r, a, P>(base, in, at);
+    row_load<r - a, P>(alpha, at, in, d);
+    const FV<P> sr = row_sum<r - a, P>(d, in);
+    s = (a == 0) ? vmul(hA[0], sr) : vfma(hA[a], sr, s);
+    if constexpr (a < r) block2_fixed<r, a + 1, P, NA>(alpha, base, in, hA, s);
 }
 
 /* planes C..R of a fully unrolled 3-D block of budget R */
-template <int R, int C, int P>
+template <int R, int C, int P, int NA>
 __device__ __forceinline__ void block3_planes(const float *__restrict__ alpha, const uint32_t (&base)[P],
-                                              const Inner<P> &in, FV<P> &s)
+                                              const Inner<P> &in, const FV<P> (&hA)[NA], FV<P> &s)
 {
     uint32_t sb[P];
     FV<P> s2;
-#pragma unroll
-    for (int p = 0; p < P; ++p) sb[p] = base[p] + coff_reg(R, C) + cell_at(in.TC[p], C) * blk2_reg(R - C);
-    block2_fixed<R - C, P>(alpha, sb, in, s2);
+    plane_at<R, C, P>(base, in, sb);
+    block2_fixed<R - C, 0, P, NA>(alpha, sb, in, hA, s2);
     s = (C == 0) ? vmul(in.hC(0), s2) : vfma(in.hC(C), s2, s);
-    if constexpr (C < R) block3_planes<R, C + 1, P>(alpha, base, in, s);
+    if constexpr (C < R) block3_planes<R, C + 1, P, NA>(alpha, base, in, hA, s);
+}
+
+/* Small blocks in two passes, every row loaded before the first is summed
+ * (in the order of block3_planes, so the results are the same bits).  The
+ * walk is bound by the latency of its gathers at 16 warps per SM; with the
+ * sums in between, ptxas keeps few loads in flight.  d = 10, n = 10, 2^22
+ * points, two points per thread: 137.4 ms without, 128.8 ms for blocks of
+ * budget <= 3 (10 rows), 141.4 ms for <= 4 (15 rows: the registers run out). */
+template <int P>
+constexpr int kAhead = 3;
+template <int R, int c, int a, int i, int P, int N>
+__device__ __forceinline__ void block3_load(const float *__restrict__ alpha, const uint32_t (&base)[P],
+                                            const Inner<P> &in, RowData<P> (&d)[N])
+{
+    uint32_t sb[P], at[P];
+    plane_at<R, c, P>(base, in, sb);
+    row_at<R - c, a, P>(sb, in, at);
+    row_load<R - c - a, P>(alpha, at, in, d[i]);
+    if constexpr (a < R - c) block3_load<R, c, a + 1, i + 1, P, N>(alpha, base, in, d);
+    else if constexpr (c < R) block3_load<R, c + 1, 0, i + 1, P, N>(alpha, base, in, d);
+}
+template <int R, int c, int a, int i, int P, int N>
+__device__ __forceinline__ void block3_sum(const Inner<P> &in, const RowData<P> (&d)[N], const FV<P> (&hA)[R + 1],
+                                           FV<P> &s2, FV<P> &s)
+{
+    const FV<P> sr = row_sum<R - c - a, P>(d[i], in);
+    s2 = (a == 0) ? vmul(hA[0], sr) : vfma(hA[a], sr, s2);
+    if constexpr (a < R - c) {
+        block3_sum<R, c, a + 1, i + 1, P, N>(in, d, hA, s2, s);
+    } else {
+        s = (c == 0) ? vmul(in.hC(0), s2) : vfma(in.hC(c), s2, s);
+        if constexpr (c < R) block3_sum<R, c + 1, 0, i + 1, P, N>(in, d, hA, s2, s);
+    }
+}
+
+/* Fully unrolled 3-D block of budget R. */
+template <int R, int P>
+__device__ __forceinline__ void block3_fixed(const float *__restrict__ alpha, const uint32_t (&base)[P],
+                                             const Inner<P> &in, FV<P> &s)
+{
+    FV<P> hA[R + 1];
+#pragma unroll
+    for (int a = 0; a <= R; ++a) hA[a] = in.hA(a);
+    if constexpr (R <= kAhead<P>) {
+        constexpr int N = (R + 1) * (R + 2) / 2;
+        RowData<P> d[N];
+        FV<P> s2;
+        block3_load<R, 0, 0, 0, P, N>(alpha, base, in, d);
+        block3_sum<R, 0, 0, 0, P, N>(in, d, hA, s2, s);
+    } else {
+        block3_planes<R, 0, P, R + 1>(alpha, base, in, hA, s);
+    }
 }
 
 /* Generic sub-block of budget r (limits, r >= kNB): runtime loops. */
@@ -253,30 +370,21 @@ __device__ __forceinline__ void block2_generic(const float *__restrict__ alpha, 
                 yA.set(p, y);
             }
         }
-        const int rl = min(r - a, limB) + 1;
-        const uint32_t plen = (1u << (rl - 1)) * (uint32_t)SG_PATH_WIDTH(rl);
-        FV<P> yB, sr = FV<P>::all(0.0f);
-        uint32_t rb[P];
+        const int L = min(r - a, limB);
+        const uint32_t plen = SG_POLE_SLOTS(L);
+        FV<P> sr;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            yB.set(p, xB[p]);
-            /* path of the finest cell t_L = floor(x_B 2^L), exact */
-            rb[p] = base[p] + aoff + tA[p] * plen +
-                    (uint32_t)(xB[p] * (float)(1u << (rl - 1))) * (uint32_t)SG_PATH_WIDTH(rl);
-        }
-        for (int b = 0; b < rl; ++b) {
-            if (b) {
-#pragma unroll
-                for (int p = 0; p < P; ++p) {
-                    float y = yB.get(p);
-                    (void)step_y(y);
-                    yB.set(p, y);
-                }
+            const float *pole = alpha + (base[p] + aoff + tA[p] * plen);
+            if (L == 0) {
+                sr.set(p, __fmul_rn(hat_of(xB[p]), __ldg(pole)));
+            } else {
+                /* cell of level 1, or half of a cell of level L, and the
+                 * position in it (exact) */
+                const float t = xB[p] * (float)(L == 1 ? 2u : 2u << L), f = truncf(t), y = t - f;
+                const float2 w = __ldg(reinterpret_cast<const float2 *>(pole + 2 * (uint32_t)f));
+                sr.set(p, L == 1 ? fmaf(hat_of(y), w.y, __fmul_rn(hat_of(xB[p]), w.x)) : fmaf(y, w.y, w.x));
             }
-            FV<P> v;
-#pragma unroll
-            for (int p = 0; p < P; ++p) v.set(p, __ldg(alpha + rb[p] + b));
-            sr = vfma(hats(yB), v, sr);
         }
         s = vfma(hasA ? hats(yA) : FV<P>::all(1.0f), sr, s);
         aoff += (1u << a) * plen;
@@ -284,14 +392,19 @@ __device__ __forceinline__ void block2_generic(const float *__restrict__ alpha, 
 }
 
 /* Sub-block of budget r: unrolled (r within the limits, r < kNB) or generic. */
-template <int D, int P>
-__device__ __forceinline__ void block2_any(const EvalArgs &A, int r, const Inner<P> &in, const float (&xA)[P],
+template <int D, int P, typename GA>
+__device__ __forceinline__ void block2_any(const GA &A, int r, const Inner<P> &in, const float (&xA)[P],
                                            const float (&xB)[P], const uint32_t (&base)[P], FV<P> &s)
 {
     if (D >= 2 && r <= A.lim2) {
         switch (r) {
-#define SG_BLK2(RR) \
-    case RR: block2_fixed<RR, P>(A.alpha, base, in, s); return;
+#define SG_BLK2(RR)                                                          \
+    case RR: {                                                               \
+        FV<P> hA[RR + 1];                                                    \
+        _Pragma("unroll") for (int a = 0; a <= RR; ++a) hA[a] = in.hA(a);    \
+        block2_fixed<RR, 0, P, RR + 1>(A.alpha, base, in, hA, s);            \
+        return;                                                              \
+    }
             SG_BLK2(0) SG_BLK2(1) SG_BLK2(2) SG_BLK2(3) SG_BLK2(4)
             SG_BLK2(5) SG_BLK2(6) SG_BLK2(7) SG_BLK2(8) SG_BLK2(9)
 #undef SG_BLK2
@@ -302,26 +415,26 @@ __device__ __forceinline__ void block2_any(const EvalArgs &A, int r, const Inner
 }
 
 /* Sum over the block of budget R at `base` for every point. */
-template <int D, int P, int BL>
-__device__ __forceinline__ void block_sum(const EvalArgs &A, int R, const Inner<P> &in, const float (&xC)[P],
+template <int D, int P, typename GA>
+__device__ __forceinline__ void block_sum(const GA &A, int R, const Inner<P> &in, const float (&xC)[P],
                                           const float (&xA)[P], const float (&xB)[P], const uint32_t (&base)[P],
                                           FV<P> &s)
 {
     if constexpr (D >= 3) {
-        if (R <= kRFof<BL> && R <= A.lim3) {
+        if (R <= kRFof<D> && R <= A.lim3) {
             switch (R) {
-            case 0: block3_planes<0, 0, P>(A.alpha, base, in, s); return;
-            case 1: block3_planes<1, 0, P>(A.alpha, base, in, s); return;
-            case 2: block3_planes<2, 0, P>(A.alpha, base, in, s); return;
-            case 3: block3_planes<3, 0, P>(A.alpha, base, in, s); return;
-            case 4: block3_planes<4, 0, P>(A.alpha, base, in, s); return;
+            case 0: block3_fixed<0, P>(A.alpha, base, in, s); return;
+            case 1: block3_fixed<1, P>(A.alpha, base, in, s); return;
+            case 2: block3_fixed<2, P>(A.alpha, base, in, s); return;
+            case 3: block3_fixed<3, P>(A.alpha, base, in, s); return;
+            case 4: block3_fixed<4, P>(A.alpha, base, in, s); return;
             case 5:
-                if constexpr (kRFof<BL> > 5) {
-                    block3_planes<5, 0, P>(A.alpha, base, in, s);
+                if constexpr (kRFof<D> > 5) {
+                    block3_fixed<5, P>(A.alpha, base, in, s);
                     return;
                 }
                 [[fallthrough]];
-            default: block3_planes<kRFof<BL>, 0, P>(A.alpha, base, in, s); return;
+            default: block3_fixed<kRFof<D>, P>(A.alpha, base, in, s); return;
             }
         }
     }
@@ -362,20 +475,85 @@ __device__ __forceinline__ void block_sum(const EvalArgs &A, int R, const Inner<
 template <int D>
 constexpr int kUpper = D >= 6 ? (D - 5 < 7 ? D - 5 : 7) : 0;
 
-/* The walk's block range of a split evaluation: blocks are numbered in
- * walk order; only [lo, hi) are summed (all of them when !partial). */
+/* Segments of the sum (sg_layout.h), as block-layout offsets compared with
+ * the walk's running offset `cur`.  The walk has no registers to spare, so it
+ * carries only the end of the current segment and the start of the warp's
+ * range (several warps may share a sum); the rest lives in local memory and is touched once per segment by a function that
+ * is not inlined (inlined, its registers cost 9 % at d = 10, n = 10). */
 struct Range {
-    uint32_t leaf, lo, hi;
-    bool partial;
+    uint32_t next; /* end of the current segment, 0xFFFFFFFF: none follows   */
+    uint32_t lo;   /* first offset of the warp's range, 0xFFFFFFFF: all done */
+};
+template <int P>
+struct Tail {
+    const uint32_t *bounds;
+    int s, end, nseg, emit;           /* current segment, end of the warp's own */
+    float part[2][P], total[2][P];    /* compensated sums                       */
+    float *out[P];                    /* shared sums: the points in part_out, or NULL */
+    int64_t stride;
+    bool valid[P], nan_in[P];
 };
 
-/* largest budget of an unrolled leaf subtree: of the last prefix dim
- * (kLGof, per points per thread under the wide preset: two points need
- * twice the registers), of the last two (kLG2) */
-template <int P, int BL>
-constexpr int kLGof = BL == 0 ? (P == 1 ? SG_EVAL_MAX_LEAF_P1 : SG_EVAL_MAX_LEAF_P2) : 3;
+template <int P>
+__device__ __forceinline__ void fold(float (&acc)[2][P], FV<P> v)
+{
+    FV<P> s, c;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        s.set(p, acc[0][p]);
+        c.set(p, acc[1][p]);
+    }
+    kahan_add(s, c, v);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        acc[0][p] = s.get(p);
+        acc[1][p] = c.get(p);
+    }
+}
+
+template <int P>
+__device__ __forceinline__ FV<P> take(float (&acc)[2][P])
+{
+    FV<P> s, c;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        s.set(p, acc[0][p]);
+        c.set(p, acc[1][p]);
+        acc[0][p] = acc[1][p] = 0.0f;
+    }
+    return vsub(s, c);
+}
+
+/* Ends the current segment, whose sum is v; returns the next segment's end. */
+template <int P>
+__device__ __noinline__ uint32_t close_segment(Tail<P> *t, FV<P> v)
+{
+    const int s = t->s++;
+    int k = s;
+    bool whole = true;
+    if (t->emit != SG_EMIT_SEGS) {
+        fold<P>(t->part, v);
+        whole = (s + 1) % SG_SEG_PER_PART == 0 || s + 1 == t->nseg;
+        if (whole) {
+            v = take<P>(t->part);
+            k = s / SG_SEG_PER_PART;
+            if (t->emit == SG_EMIT_SUM) fold<P>(t->total, v);
+        }
+    }
+    if (whole && t->emit != SG_EMIT_SUM) {
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (t->out[p])
+                t->out[p][k * t->stride] = t->valid[p] ? v.get(p) : (t->nan_in[p] ? __int_as_float(0x7fc00000) : 0.0f);
+    }
+    return s + 2 < t->nseg ? __ldg(t->bounds + s + 2) : 0xFFFFFFFFu;
+}
+
+/* largest budget of an unrolled leaf subtree of the last two prefix dims (of
+ * the last one: SG_EVAL_MAX_LEAF) */
 constexpr int kLG2 = SG_EVAL_MAX_LEAF2;
-static_assert(SG_EVAL_MAX_LEAF_P1 <= 5 && SG_EVAL_MAX_LEAF_P2 <= 5 && kLG2 <= 3,
+static_assert(kLG2 == SG_SEG_UNIT_BUDGET, "segments start outside the unrolled subtrees");
+static_assert(SG_EVAL_MAX_LEAF <= 5 && kLG2 <= 3,
               "the walk's jump tables cover leaf budgets 0..5 and 0..3");
 /* unrolled subtrees are instantiated for d <= kMaxUnrollD only (their code
  * grows with d; grids of more dims keep the loop) */
@@ -396,8 +574,8 @@ __device__ __forceinline__ void step_all(FV<P> &y, uint32_t (&ix)[P])
 
 /* Levels l = L..B of the last prefix dim and their 3-D blocks of budget
  * B - l, fully unrolled (every shape regular: B within the limits). */
-template <int D, int P, int B, int L>
-__device__ __forceinline__ void leaf_group(const EvalArgs &A, uint32_t &cur, const Inner<P> &in, const FV<P> &pin,
+template <int D, int P, int B, int L, typename GA>
+__device__ __forceinline__ void leaf_group(const GA &A, uint32_t &cur, const Inner<P> &in, const FV<P> &pin,
                                            FV<P> &y, uint32_t (&ix)[P], FV<P> &acc)
 {
     if constexpr (L > 0) step_all<P>(y, ix);
@@ -408,7 +586,7 @@ __device__ __forceinline__ void leaf_group(const EvalArgs &A, uint32_t &cur, con
 #pragma unroll
     for (int p = 0; p < P; ++p) base[p] = cur + ix[p] * blk;
     cur += blk << (A.nm1 - R);
-    block3_planes<R, 0, P>(A.alpha, base, in, s);
+    block3_fixed<R, P>(A.alpha, base, in, s);
     acc = vfma(vmul(pin, hats(y)), s, acc);
     if constexpr (L < B) leaf_group<D, P, B, L + 1>(A, cur, in, pin, y, ix, acc);
 }
@@ -426,8 +604,8 @@ __device__ __forceinline__ FV<P> load_y(const float *sx, int K, int tid)
 /* Levels l = L..B of prefix dim K = D-5, each followed by the unrolled
  * leaf group of dim D-4 with budget B - l (one compensated add per group,
  * as in the walk). */
-template <int D, int K, int P, int B, int L>
-__device__ __forceinline__ void leaf_group2(const EvalArgs &A, const float *sx, int tid, uint32_t &cur,
+template <int D, int K, int P, int B, int L, typename GA>
+__device__ __forceinline__ void leaf_group2(const GA &A, const float *sx, int tid, uint32_t &cur,
                                             const Inner<P> &in, const FV<P> &pin, FV<P> &y, uint32_t (&ix)[P],
                                             FV<P> &sum, FV<P> &comp)
 {
@@ -444,14 +622,52 @@ __device__ __forceinline__ void leaf_group2(const EvalArgs &A, const float *sx, 
 }
 
 /* Walk over prefix dim K (K <= D-4); children of depth D-4 are blocks.
- * M = mode: bit 0 (SPLIT) = the caller may ask for a block range (batched
- * launches), bits 1.. (BL) = the blocking preset. */
-template <int D, int K, int P, int M>
+ * Segments start at iterations of the loops at depth K <= D-5 (D = 4: of its
+ * only loop), so subtrees outside the warp's range are skipped there by their
+ * extents, and segments are closed where the innermost of those loops
+ * starts an iteration (every outer iteration starts one of it). */
+template <int D, int K, int P, bool SH>
 struct Walk {
-    static constexpr bool SPLIT = (M & 1) != 0;
-    static constexpr int BL = M >> 1;
-    static __device__ __forceinline__ void run(const EvalArgs &A, const float *sx, int tid, int budget,
-                                               uint32_t &cur, Range &rg, const Inner<P> &in, const float (&xC)[P],
+    static constexpr bool kLoop = D == 4 ? K == 0 : K + 5 <= D;  /* may skip  */
+    static constexpr bool kClose = D == 4 ? K == 0 : K + 5 == D; /* closes    */
+
+    /* child of budget `left` lies before the range (or the range is done):
+     * step over it */
+    template <typename GA>
+    static __device__ __forceinline__ bool skip(const GA &A, const Range &rg, int left, uint32_t &cur)
+    {
+        if constexpr (kLoop && SH) {
+            if (cur < rg.lo) {
+                const uint32_t ext = __ldg(A.seg + (K + 1) * (A.nm1 + 1) + left);
+                if (cur + ext <= rg.lo) {
+                    cur += ext;
+                    return true;
+                }
+            }
+        }
+        return false;
+    }
+    /* closes the segments that end at or before cur; true when the warp's
+     * own are all closed */
+    static __device__ __forceinline__ bool close(Range &rg, Tail<P> *tl, uint32_t cur, FV<P> &sum, FV<P> &comp)
+    {
+        while (cur >= rg.next) {
+            rg.next = close_segment<P>(tl, vsub(sum, comp));
+            sum = comp = FV<P>::all(0.0f);
+            if constexpr (SH) {
+                if (tl->s >= tl->end) {
+                    rg.lo = rg.next = 0xFFFFFFFFu;
+                    return true;
+                }
+            }
+        }
+        return false;
+    }
+
+    template <typename GA>
+    static __device__ __forceinline__ void run(const GA &A, const float *sx, int tid, int budget,
+                                               uint32_t &cur, Range &rg, Tail<P> *tl, const Inner<P> &in,
+                                               const float (&xC)[P],
                                                const float (&xA)[P], const float (&xB)[P], const FV<P> &pin,
                                                const uint32_t (&ixin)[P], FV<P> &sum, FV<P> &comp)
     {
@@ -468,36 +684,33 @@ struct Walk {
                 ws[(1 * P + p) * kThreads] = __uint_as_float(ixin[p]);
                 ws[(2 * P + p) * kThreads] = pin.get(p);
             }
+#pragma unroll 1
             for (int l = 0; l <= lmax; ++l) {
-                FV<P> y, pp;
-                uint32_t ix[P];
+                FV<P> y, pp, yn;
+                uint32_t ix[P], ixn[P];
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     y.set(p, ws[(0 * P + p) * kThreads]);
-                    ix[p] = __float_as_uint(ws[(1 * P + p) * kThreads]);
+                    ix[p] = ixn[p] = __float_as_uint(ws[(1 * P + p) * kThreads]);
                     pp.set(p, ws[(2 * P + p) * kThreads]);
                 }
-                if (l) {
-                    step_all<P>(y, ix);
+                /* the next level's state */
+                yn = y;
+                step_all<P>(yn, ixn);
 #pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        ws[(0 * P + p) * kThreads] = y.get(p);
-                        ws[(1 * P + p) * kThreads] = __uint_as_float(ix[p]);
-                    }
+                for (int p = 0; p < P; ++p) {
+                    ws[(0 * P + p) * kThreads] = yn.get(p);
+                    ws[(1 * P + p) * kThreads] = __uint_as_float(ixn[p]);
                 }
-                if (SPLIT && rg.partial) {
-                    const uint32_t *w = A.walk + 2 * ((K + 1) * (A.nm1 + 1) + (budget - l));
-                    const uint32_t nb = __ldg(w);
-                    if (rg.leaf + nb <= rg.lo || rg.leaf >= rg.hi) {
-                        rg.leaf += nb;
-                        cur += __ldg(w + 1);
-                        continue;
-                    }
-                }
+                if (skip(A, rg, budget - l, cur)) continue;
                 const FV<P> pn = vmul(pp, hats(y));
-                Walk<D, K + 1, P, M>::run(A, sx, tid, budget - l, cur, rg, in, xC, xA, xB, pn, ix, sum, comp);
+                Walk<D, K + 1, P, SH>::run(A, sx, tid, budget - l, cur, rg, tl, in, xC, xA, xB, pn, ix, sum, comp);
             }
             return;
+        }
+        if constexpr (kClose && D > 4) {
+            /* the first iteration's close, before the unrolled forms below */
+            if (close(rg, tl, cur, sum, comp)) return;
         }
         const int lmax = min(A.lim[K], budget);
         FV<P> y = load_y<P>(sx, K, tid);
@@ -506,8 +719,7 @@ struct Walk {
 #pragma unroll
         for (int p = 0; p < P; ++p) ix[p] = ixin[p];
         if constexpr (D <= kMaxUnrollD && K + 1 == D - 4) {
-            if (!(SPLIT && rg.partial) && budget <= kLG2 && budget <= A.lim[K] && budget <= A.lim[K + 1] &&
-                budget <= A.lim3) {
+            if (budget <= kLG2 && budget <= A.lim[K] && budget <= A.lim[K + 1] && budget <= A.lim3) {
                 switch (budget) {
                 case 0: leaf_group2<D, K, P, 0, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
                 case 1: leaf_group2<D, K, P, 1, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
@@ -519,17 +731,17 @@ struct Walk {
             }
         }
         if constexpr (D <= kMaxUnrollD && K == D - 4) {
-            if (!(SPLIT && rg.partial) && budget <= kLGof<P, BL> && budget <= A.lim[K] && budget <= A.lim3) {
+            if (budget <= SG_EVAL_MAX_LEAF && budget <= A.lim[K] && budget <= A.lim3) {
                 switch (budget) {
                 case 0: leaf_group<D, P, 0, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 1: leaf_group<D, P, 1, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 2: leaf_group<D, P, 2, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 3: leaf_group<D, P, 3, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 4:
-                    if constexpr (kLGof<P, BL> >= 4) leaf_group<D, P, 4, 0>(A, cur, in, pin, y, ix, acc);
+                    if constexpr (SG_EVAL_MAX_LEAF >= 4) leaf_group<D, P, 4, 0>(A, cur, in, pin, y, ix, acc);
                     break;
                 case 5:
-                    if constexpr (kLGof<P, BL> >= 5) leaf_group<D, P, 5, 0>(A, cur, in, pin, y, ix, acc);
+                    if constexpr (SG_EVAL_MAX_LEAF >= 5) leaf_group<D, P, 5, 0>(A, cur, in, pin, y, ix, acc);
                     break;
                 default: break;
                 }
@@ -537,18 +749,17 @@ struct Walk {
                 return;
             }
         }
-        for (int l = 0; l <= lmax; ++l) {
-            if (l) step_all<P>(y, ix);
-            if (SPLIT && rg.partial) {
-                /* the child subtree (depth K+1, budget - l) holds blocks
-                 * [leaf, leaf + nb): skip it whole when outside [lo, hi) */
-                const uint32_t *w = A.walk + 2 * ((K + 1) * (A.nm1 + 1) + (budget - l));
-                const uint32_t nb = __ldg(w);
-                if (rg.leaf + nb <= rg.lo || rg.leaf >= rg.hi) {
-                    rg.leaf += nb;
-                    cur += __ldg(w + 1);
-                    continue;
+#pragma unroll 1
+        for (int l = 0; l <= lmax; ++l, step_all<P>(y, ix)) {
+            if (skip(A, rg, budget - l, cur)) continue;
+            if constexpr (kClose) {
+                if constexpr (D == 4) {
+                    if (cur >= rg.next) {
+                        kahan_add(sum, comp, acc);
+                        acc = FV<P>::all(0.0f);
+                    }
                 }
+                if (close(rg, tl, cur, sum, comp)) return;
             }
             const FV<P> pn = vmul(pin, hats(y));
             if constexpr (K == D - 4) {
@@ -559,11 +770,10 @@ struct Walk {
 #pragma unroll
                 for (int p = 0; p < P; ++p) base[p] = cur + ix[p] * blk;
                 cur += blk << (A.nm1 - R);
-                if (SPLIT) ++rg.leaf;
-                block_sum<D, P, BL>(A, R, in, xC, xA, xB, base, s);
+                block_sum<D, P>(A, R, in, xC, xA, xB, base, s);
                 acc = vfma(pn, s, acc);
             } else {
-                Walk<D, K + 1, P, M>::run(A, sx, tid, budget - l, cur, rg, in, xC, xA, xB, pn, ix, sum, comp);
+                Walk<D, K + 1, P, SH>::run(A, sx, tid, budget - l, cur, rg, tl, in, xC, xA, xB, pn, ix, sum, comp);
             }
         }
         if constexpr (K == D - 4) kahan_add(sum, comp, acc);
@@ -572,12 +782,12 @@ struct Walk {
 
 /* Evaluates this thread's points first, first + 32, ..., first + 32(P-1)
  * (those below `end`) against grid A; sx is this CTA's shared coordinate
- * buffer, shat its shared hats of dims A and C. */
-template <int D, int P, int M>
-__device__ __forceinline__ void eval_points(const EvalArgs &A, float *sx, FV<P> *shat, int tid, int64_t first,
-                                            int64_t end, int part)
+ * buffer, shat its shared hats of dims A and C; share = which of the
+ * A.nshare shares of the segments this warp adds up. */
+template <int D, int P, bool SH, typename GA>
+__device__ __forceinline__ void eval_points(const EvalArgs &A, const GA &G, float *sx, FV<P> *shat, int tid, int64_t first,
+                                            int64_t end, int share)
 {
-    constexpr bool SPLIT = (M & 1) != 0;
     float xC[P], xA[P], xB[P];
     bool valid[P], nan_in[P];
 #pragma unroll
@@ -609,15 +819,20 @@ __device__ __forceinline__ void eval_points(const EvalArgs &A, float *sx, FV<P> 
     }
 
     Inner<P> in;
-    in.sh = shat + tid;
+    in.sh = (uint32_t)__cvta_generic_to_shared(shat + tid);
     FV<P> *const shw = shat + tid;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         float y = xB[p];
+        in.xB.set(p, y);
+        in.hB[0].set(p, hat_of(y));
+        (void)step_y(y);
+        in.hB[1].set(p, hat_of(y));
+        (void)step_y(y);
 #pragma unroll
-        for (int j = 0; j < kNB; ++j) {
-            if (j) (void)step_y(y);
-            in.hB[j].set(p, hat_of(y));
+        for (int j = 0; j < kYReg; ++j) {
+            (void)step_y(y);
+            in.yB[j].set(p, y);
         }
         in.TB[p] = (uint32_t)(xB[p] * (float)(1u << kTB));
         in.TA[p] = (uint32_t)(xA[p] * (float)(1u << kTB));
@@ -654,6 +869,8 @@ __device__ __forceinline__ void eval_points(const EvalArgs &A, float *sx, FV<P> 
         }
     }
 
+    asm volatile("" ::: "memory"); /* the hats are stored before lds_hat reads them */
+
     FV<P> sum = FV<P>::all(0.0f), comp = FV<P>::all(0.0f);
     uint32_t cur = 0;
     if constexpr (D >= 4) {
@@ -662,17 +879,38 @@ __device__ __forceinline__ void eval_points(const EvalArgs &A, float *sx, FV<P> 
 #pragma unroll
         for (int p = 0; p < P; ++p) ix[p] = 0;
         Range rg;
-        rg.leaf = 0;
-        rg.partial = SPLIT && A.nparts > 1;
-        rg.lo = rg.partial ? A.split[part] : 0u;
-        rg.hi = rg.partial ? A.split[part + 1] : 0xFFFFFFFFu;
-        Walk<D, 0, P, M>::run(A, sx, tid, A.nm1, cur, rg, in, xC, xA, xB, pin, ix, sum, comp);
+        Tail<P> tl;
+        tl.bounds = A.seg + (D - 2) * (A.nm1 + 1);
+        tl.s = share * A.nseg / A.nshare;
+        tl.end = (share + 1) * A.nseg / A.nshare;
+        tl.nseg = A.nseg;
+        tl.emit = A.emit;
+        tl.stride = A.num_evals;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            tl.out[p] = first + 32 * p < end ? A.part_out + first + 32 * p : nullptr;
+            tl.valid[p] = valid[p];
+            tl.nan_in[p] = nan_in[p];
+            tl.part[0][p] = tl.part[1][p] = tl.total[0][p] = tl.total[1][p] = 0.0f;
+        }
+        rg.lo = tl.s > 0 ? __ldg(tl.bounds + tl.s) : 0u;
+        rg.next = tl.s + 1 < A.nseg ? __ldg(tl.bounds + tl.s + 1) : 0xFFFFFFFFu;
+        Walk<D, 0, P, SH>::run(G, sx, tid, A.nm1, cur, rg, &tl, in, xC, xA, xB, pin, ix, sum, comp);
+        if (A.nseg > 1) {
+            while (tl.s < tl.end) {
+                (void)close_segment<P>(&tl, vsub(sum, comp));
+                sum = comp = FV<P>::all(0.0f);
+            }
+            if (A.emit != SG_EMIT_SUM) return;
+            sum = take<P>(tl.total);
+            comp = FV<P>::all(0.0f);
+        }
     } else {
         uint32_t base[P];
         FV<P> s;
 #pragma unroll
         for (int p = 0; p < P; ++p) base[p] = 0;
-        block_sum<D, P, (M >> 1)>(A, A.nm1, in, xC, xA, xB, base, s);
+        block_sum<D, P>(G, A.nm1, in, xC, xA, xB, base, s);
         kahan_add(sum, comp, s);
     }
 
@@ -682,10 +920,7 @@ __device__ __forceinline__ void eval_points(const EvalArgs &A, float *sx, FV<P> 
         const int64_t i = first + 32 * p;
         if (i < end) {
             const float r = valid[p] ? res.get(p) : (nan_in[p] ? __int_as_float(0x7fc00000) : 0.0f);
-            if (SPLIT && A.nparts > 1)
-                A.part_out[(int64_t)part * A.num_evals + i] = r;
-            else
-                A.out[A.perm ? A.perm[i] : i] = r;
+            A.out[A.perm ? A.perm[i] : i] = r;
         }
     }
 }
@@ -696,121 +931,115 @@ template <int D, int P>
 constexpr int kSmemBytes = kHatSlots * kThreads * (int)sizeof(FV<P>) + (D >= 4 ? D - 3 : 1) * P * kThreads * 4 +
                            kUpper<D> * 3 * P * kThreads * 4;
 
-/* blocking presets instantiated for dimension D: both where the leaf
- * groups and 3-D blocks exist (3 <= D <= kMaxUnrollD); elsewhere one,
- * kBaseBL<D>: medium above kMaxUnrollD (no leaf groups; the wide preset's
- * larger 3-D blocks only add spills to those kernels' large walk state),
- * wide below 3 (no 3-D blocks: the presets are the same code) */
-template <int D>
-constexpr int kBlockings = (D >= 3 && D <= kMaxUnrollD) ? SG_EVAL_BLOCKINGS : 1;
-template <int D>
-constexpr int kBaseBL = D > kMaxUnrollD ? 1 : 0;
-static_assert(SG_EVAL_BLOCKINGS == 2, "presets: wide (0) and medium (1)");
-
-template <int D, int P, int BL>
-__global__ void __launch_bounds__(kThreads, (P == 2 ? 2 : 3)) k_evaluate(const EvalArgs A)
+template <int D, int P>
+__global__ void __launch_bounds__(kThreads, 2) k_evaluate(const EvalArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_ev[];
     FV<P> *shat = reinterpret_cast<FV<P> *>(smem_ev);
     float *sx = reinterpret_cast<float *>(smem_ev + kHatSlots * kThreads * sizeof(FV<P>));
     const int tid = threadIdx.x;
     const int64_t warp = (blockIdx.x * (int64_t)kThreads + tid) >> 5;
-    eval_points<D, P, 2 * BL>(A, sx, shat, tid, warp * (32 * P) + (tid & 31), A.num_evals, 0);
+    eval_points<D, P, false>(A, A, sx, shat, tid, warp * (32 * P) + (tid & 31), A.num_evals, 0);
 }
 
 /* Many grids of the same dimension in one launch: CTA b evaluates the
  * kThreads*P points of grid items[b].x & (2^29-1) starting at point
- * items[b].y; bits 29..31 of items[b].x select the part of a split sum. */
-template <int D, int P, int BL>
-__global__ void __launch_bounds__(kThreads, (P == 2 ? 2 : 3))
-    k_evaluate_batch(const EvalArgs *__restrict__ grids, const int2 *__restrict__ items)
+ * items[b].y.  SH: sums may be shared, bits 29..31 of items[b].x select the
+ * share of the segments; without a table of grids the launch is for grid
+ * `one`, whose warps are numbered share by share (warps of one share are
+ * neighbours: they read the same part of the grid). */
+template <int D, int P, bool SH>
+__global__ void __launch_bounds__(kThreads, 2)
+    k_evaluate_batch(const EvalArgs *__restrict__ grids, const int2 *__restrict__ items, const EvalArgs one)
 {
     extern __shared__ __align__(16) unsigned char smem_ev[];
     FV<P> *shat = reinterpret_cast<FV<P> *>(smem_ev);
     float *sx = reinterpret_cast<float *>(smem_ev + kHatSlots * kThreads * sizeof(FV<P>));
     __shared__ EvalArgs sA;
     const int tid = threadIdx.x;
-    const int2 item = items[blockIdx.x];
-    const int q = item.x & 0x1FFFFFFF, part = (int)((unsigned)item.x >> 29);
-    {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(grids + q);
+    int share = 0;
+    int64_t first, end;
+    if (SH && !grids) {
+        if (tid == 0) sA = one;
+        __syncthreads();
+        const int64_t warp = (blockIdx.x * (int64_t)kThreads + tid) >> 5, groups = (sA.num_evals + 32 * P - 1) / (32 * P);
+        share = (int)(warp / groups);
+        if (share >= sA.nshare) return;
+        first = (warp - share * groups) * (32 * P) + (tid & 31);
+        end = sA.num_evals;
+    } else {
+        const int2 item = items[blockIdx.x];
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(grids + (item.x & 0x1FFFFFFF));
         uint32_t *dst = reinterpret_cast<uint32_t *>(&sA);
         for (int w = tid; w < (int)(sizeof(EvalArgs) / 4); w += kThreads) dst[w] = src[w];
+        __syncthreads();
+        if (SH) share = (int)((unsigned)item.x >> 29);
+        first = (int64_t)item.y + (tid >> 5) * (32 * P) + (tid & 31);
+        end = min((int64_t)item.y + (int64_t)kThreads * P, sA.num_evals);
     }
-    __syncthreads();
-    const int64_t start = item.y;
-    const int64_t end = min(start + (int64_t)kThreads * P, sA.num_evals);
-    eval_points<D, P, 2 * BL + 1>(sA, sx, shat, tid, start + (tid >> 5) * (32 * P) + (tid & 31), end, part);
-}
-
-template <int D, int P, int BL>
-int launch_eval(const EvalArgs &A, void *stream)
-{
-    const int64_t per_block = (int64_t)kThreads * P;
-    const int64_t blocks = (A.num_evals + per_block - 1) / per_block;
-    if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
-    k_evaluate<D, P, BL><<<(unsigned)blocks, kThreads, kSmemBytes<D, P>, (cudaStream_t)stream>>>(A);
-    sgk_count(1);
-    return cudaGetLastError();
-}
-
-template <int D, int P, int BL>
-int launch_eval_batch(const EvalArgs *grids, const int2 *items, int nitems, void *stream)
-{
-    k_evaluate_batch<D, P, BL><<<nitems, kThreads, kSmemBytes<D, P>, (cudaStream_t)stream>>>(grids, items);
-    sgk_count(1);
-    return cudaGetLastError();
-}
-
-template <int D, int BL>
-int set_smem(void)
-{
-    int e = cudaFuncSetAttribute(k_evaluate<D, 1, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<D, 1>);
-    if (!e) e = cudaFuncSetAttribute(k_evaluate<D, 2, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<D, 2>);
-    if (!e)
-        e = cudaFuncSetAttribute(k_evaluate_batch<D, 1, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes<D, 1>);
-    if (!e)
-        e = cudaFuncSetAttribute(k_evaluate_batch<D, 2, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes<D, 2>);
-    return e;
+    const GridView view(sA);
+    eval_points<D, P, SH>(sA, view, sx, shat, tid, first, end, share);
 }
 
 } // namespace sgeval
 
-/* Lets the kernels of dimension D use their dynamic shared memory (above
- * 48 KB for d >= 8 at two points per thread) on the current device; called
- * once per device before the first launch (outside any stream capture). */
-template <int D>
-int eval_setup()
-{
-    int e = sgeval::set_smem<D, sgeval::kBaseBL<D>>();
-    if constexpr (sgeval::kBlockings<D> > 1)
-        if (!e) e = sgeval::set_smem<D, 1>();
-    return e;
-}
+/* points per thread: two, the lanes of the packed FP32x2 instructions */
+constexpr int kPts = 2;
 
-/* blocking: preset index; dimensions with one form take kBaseBL<D> */
+/* Each launcher also lets its kernel use its dynamic shared memory (above
+ * 48 KB for d >= 8) on the current device when called with no work (A or
+ * grids NULL, no items): once per device, before the first launch and outside
+ * any stream capture. */
+#if SG_EVAL_PART == 0
 template <int D>
-int eval_launch(const EvalArgs &A, int ppt, int blocking, void *stream)
+int eval_launch(const EvalArgs *A, void *stream)
 {
-    constexpr int B0 = sgeval::kBaseBL<D>;
-    if constexpr (sgeval::kBlockings<D> > 1)
-        if (blocking == 1) return ppt == 1 ? sgeval::launch_eval<D, 1, 1>(A, stream) : sgeval::launch_eval<D, 2, 1>(A, stream);
-    return ppt == 1 ? sgeval::launch_eval<D, 1, B0>(A, stream) : sgeval::launch_eval<D, 2, B0>(A, stream);
+    using namespace sgeval;
+    if (!A)
+        return cudaFuncSetAttribute(k_evaluate<D, kPts>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSmemBytes<D, kPts>);
+    const int64_t blocks = (A->num_evals + SG_EVAL_CTA_POINTS - 1) / SG_EVAL_CTA_POINTS;
+    if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+    k_evaluate<D, kPts><<<(unsigned)blocks, kThreads, kSmemBytes<D, kPts>, (cudaStream_t)stream>>>(*A);
+    sgk_count(1);
+    return cudaGetLastError();
 }
-
+#elif SG_EVAL_PART == 1
 template <int D>
-int eval_batch_launch(const EvalArgs *grids, const int2 *items, int nitems, int ppt, int blocking, void *stream)
+int eval_batch_launch(const EvalArgs *grids, const int2 *items, int nitems, void *stream)
 {
+    using namespace sgeval;
+    if (!grids)
+        return cudaFuncSetAttribute(k_evaluate_batch<D, kPts, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSmemBytes<D, kPts>);
     if (nitems <= 0) return cudaSuccess;
-    if constexpr (sgeval::kBlockings<D> > 1)
-        if (blocking == 1)
-            return ppt == 1 ? sgeval::launch_eval_batch<D, 1, 1>(grids, items, nitems, stream)
-                            : sgeval::launch_eval_batch<D, 2, 1>(grids, items, nitems, stream);
-    constexpr int B0 = sgeval::kBaseBL<D>;
-    return ppt == 1 ? sgeval::launch_eval_batch<D, 1, B0>(grids, items, nitems, stream)
-                    : sgeval::launch_eval_batch<D, 2, B0>(grids, items, nitems, stream);
+    k_evaluate_batch<D, kPts, false><<<nitems, kThreads, kSmemBytes<D, kPts>, (cudaStream_t)stream>>>(grids, items,
+                                                                                                    EvalArgs());
+    sgk_count(1);
+    return cudaGetLastError();
 }
+#else
+template <int D>
+int eval_shared_launch(const EvalArgs *grids, const int2 *items, int nitems, const EvalArgs *one, void *stream)
+{
+    using namespace sgeval;
+    constexpr bool kHas = D >= 4; /* below, every sum is one segment */
+    if (!grids && !one)
+        return kHas ? cudaFuncSetAttribute(k_evaluate_batch<D, kPts, kHas>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSmemBytes<D, kPts>)
+                    : cudaSuccess;
+    int64_t blocks = nitems;
+    if (one) {
+        const int64_t warps = (one->num_evals + 32 * kPts - 1) / (32 * kPts) * one->nshare;
+        blocks = (warps + kThreads / 32 - 1) / (kThreads / 32);
+    }
+    if (!kHas || blocks > 0x7fffffff) return cudaErrorInvalidValue;
+    if (blocks <= 0) return cudaSuccess;
+    k_evaluate_batch<D, kPts, kHas><<<(unsigned)blocks, kThreads, kSmemBytes<D, kPts>, (cudaStream_t)stream>>>(
+        one ? nullptr : grids, items, one ? *one : EvalArgs());
+    sgk_count(1);
+    return cudaGetLastError();
+}
+#endif
 
 #endif

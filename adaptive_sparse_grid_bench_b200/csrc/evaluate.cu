@@ -24,8 +24,37 @@ namespace {
 
 constexpr int kThreads = 256;
 
-/* Adds the parts of split sums in part order with Kahan compensation; CTA
- * b covers kThreads points of request items[b].x from point items[b].y
+__device__ __forceinline__ void kahan(float &s, float &c, float v)
+{
+    const float y = __fsub_rn(v, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+}
+
+/* Total of one point from what its warps wrote: the parts, or the segments
+ * part by part, in order and compensated as eval_impl.cuh adds them. */
+__device__ __forceinline__ float combine(const float *__restrict__ src, int64_t m, int nseg, int nparts, int emit)
+{
+    float s = 0.0f, c = 0.0f;
+    if (emit == SG_EMIT_PARTS) {
+        for (int k = 0; k < nparts; ++k) kahan(s, c, src[k * m]);
+        return __fsub_rn(s, c);
+    }
+    for (int k0 = 0; k0 < nseg; k0 += SG_SEG_PER_PART) {
+        float ps = 0.0f, pc = 0.0f;
+        float v[SG_SEG_PER_PART];
+#pragma unroll
+        for (int k = 0; k < SG_SEG_PER_PART; ++k) v[k] = k0 + k < nseg ? src[(k0 + k) * m] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < SG_SEG_PER_PART; ++k)
+            if (k0 + k < nseg) kahan(ps, pc, v[k]);
+        kahan(s, c, __fsub_rn(ps, pc));
+    }
+    return __fsub_rn(s, c);
+}
+
+/* CTA b covers kThreads points of request items[b].x from point items[b].y
  * (sorted positions when the request has a permutation: the sum of point i
  * goes to out[perm[i]]). */
 __global__ void __launch_bounds__(kThreads) k_combine_parts(const sg_eval_args *__restrict__ grids,
@@ -35,41 +64,65 @@ __global__ void __launch_bounds__(kThreads) k_combine_parts(const sg_eval_args *
     const sg_eval_args *A = grids + item.x;
     const int64_t m = A->num_evals, i = (int64_t)item.y + threadIdx.x;
     if (i >= m) return;
-    const int np = A->nparts;
-    const float *src = A->part_out;
-    float s = 0.0f, c = 0.0f;
-    for (int k = 0; k < np; ++k) {
-        const float y = __fsub_rn(src[k * m + i], c);
-        const float t = __fadd_rn(s, y);
-        c = __fsub_rn(__fsub_rn(t, s), y);
-        s = t;
-    }
-    A->out[A->perm ? A->perm[i] : i] = __fsub_rn(s, c);
+    A->out[A->perm ? A->perm[i] : i] = combine(A->part_out + i, m, A->nseg, A->nparts, A->emit);
 }
 
-/* compact (group-aligned) layout -> block layout: every value of level b
- * of dim B goes to slot b of the 2^(L-b) paths of its pole that pass
- * through its cell */
-__global__ void k_repack(const float *__restrict__ src, float *__restrict__ dst,
-                         const sg_repack *__restrict__ rp, int64_t nsub)
+__global__ void __launch_bounds__(64) k_combine_one(const float *__restrict__ src, const int32_t *__restrict__ perm,
+                                                    float *__restrict__ out, int64_t m, int nseg, int nparts, int emit)
 {
-    /* one warp per subspace: most subspaces hold a few values, and a warp
-     * per subspace keeps many descriptor loads in flight */
+    const int64_t i = blockIdx.x * (int64_t)64 + threadIdx.x;
+    if (i < m) out[perm ? perm[i] : i] = combine(src + i, m, nseg, nparts, emit);
+}
+
+/* compact (group-aligned) layout -> block layout, one warp per piece of
+ * kRepackPiece outputs of a row.  An output is a point's slot or pair of the
+ * row (sg_layout.h): the surplus (L = 0), the surpluses of levels 0 and 1
+ * (L = 1), or, on half h of a cell of level L, the value at the half's left
+ * end and the change to its right end of the sum over the L+1 levels.  Level
+ * b's cell is h >> (L+1-b); the hat's value at the left end is a multiple of
+ * 2^(b-L) and its change over the half is +-2^(b-L), so both sums are taken in
+ * FP64 from the surpluses, level by level, and rounded once. */
+constexpr int kRepackPiece = 1024;
+
+__global__ void __launch_bounds__(256) k_repack(const float *__restrict__ src, float *__restrict__ dst,
+                                                const sg_repack *__restrict__ rows,
+                                                const uint32_t *__restrict__ offs, int64_t nitems, int pieces)
+{
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < nsub; q += nw) {
-        const sg_repack r = rp[q];
-        const int ab = r.a + r.b, cab = r.c + ab;
-        const int rep = r.L - r.b; /* the value fills slot b of 2^rep paths */
-        const int n = 1 << (r.s + rep);
-        const uint32_t w = (uint32_t)SG_PATH_WIDTH(r.L + 1);
-        for (int f = threadIdx.x & 31; f < n; f += 32) {
-            const uint32_t e = (uint32_t)f >> rep, j = (uint32_t)f & ((1u << rep) - 1u);
-            const uint32_t I = e >> cab;
-            const uint32_t tc = (e >> ab) & ((1u << r.c) - 1u);
-            const uint32_t ta = (e >> r.b) & ((1u << r.a) - 1u);
-            const uint32_t tb = e & ((1u << r.b) - 1u);
-            const uint32_t path = (tb << rep) | j; /* finest cell t_L of the path */
-            dst[r.dst + I * r.blk + tc * r.sub + ta * r.plen + path * w] = src[r.src + e];
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < nitems; w += nw) {
+        const sg_repack r = rows[w / pieces];
+        const uint32_t first = (uint32_t)(w % pieces) * kRepackPiece;
+        const int L = r.L, lg = L == 0 ? 0 : (L == 1 ? 1 : L + 1);
+        const uint32_t n = 1u << (r.s + lg);
+        const uint32_t last = min(n, first + kRepackPiece);
+        const uint32_t *o = offs + r.src;
+        for (uint32_t f = first + (threadIdx.x & 31); f < last; f += 32) {
+            const uint32_t h = f & ((1u << lg) - 1u), e = f >> lg;
+            const uint32_t I = e >> (r.c + r.a);
+            const uint32_t tc = (e >> r.a) & ((1u << r.c) - 1u);
+            const uint32_t ta = e & ((1u << r.a) - 1u);
+            float *out = dst + (r.dst + I * r.blk + tc * r.sub + ta * r.plen + (L ? 2 * h : 0));
+            if (L == 0) {
+                *out = src[o[0] + e];
+            } else if (L == 1) {
+                *reinterpret_cast<float2 *>(out) = make_float2(src[o[0] + e], src[o[1] + f]);
+            } else {
+                double v = 0.0, dv = 0.0;
+#pragma unroll 4
+                for (int b = 0; b <= L; ++b) {
+                    const int u = L + 1 - b; /* halves of level L per cell of level b: 2^u */
+                    const uint32_t m = h & ((1u << u) - 1u), half = 1u << (u - 1);
+                    const double a = (double)src[o[b] + (e << b) + (h >> u)];
+                    const double step = 1.0 / (double)half; /* 2^(b-L) */
+                    /* the hat is 0 at the left end of its cell: no product, so
+                     * an infinite surplus leaves the cell's ends alone */
+                    if (m) v += a * ((m < half ? (double)m : (double)(2 * half - m)) * step);
+                    dv += m < half ? a * step : -(a * step);
+                }
+                float2 p = make_float2(__double2float_rn(v), __double2float_rn(dv));
+                if (!(fabsf(p.x) <= 3.402823466e38f)) p.y = 0.0f; /* inf or NaN over the whole half */
+                *reinterpret_cast<float2 *>(out) = p;
+            }
         }
     }
 }
@@ -80,12 +133,20 @@ struct SortGeom {
     int key_bits; /* total Morton bits                   */
 };
 
+/* Morton key over the leading dims.  The two innermost dims only select a
+ * place inside a block of a few cache lines, so for d > 5 all bits go to the
+ * others, where they make a warp's points share blocks (d = 10, n = 10: 11.47
+ * -> 10.71 ms per 2^18 points, 143.1 -> 141.9 ms per 2^22; without dim d-2
+ * alone 10.93 and 142.1).  Up to d = 5 most subspaces lie in the inner dims. */
+__device__ __forceinline__ int key_dims(int d) { return d > 5 ? d - 2 : d; }
+
 __device__ __forceinline__ uint32_t morton_key(const float *x, int d, int key_bits)
 {
+    const int dk = key_dims(d);
     uint32_t key = 0;
     for (int b = 0; b < key_bits; ++b) {
-        const int k = b % d;
-        const int lvl = b / d; /* bit lvl (from the top) of coordinate k */
+        const int k = b % dk;
+        const int lvl = b / dk; /* bit lvl (from the top) of coordinate k */
         float v = x[k];
         v = v >= 0.0f ? (v < 1.0f ? v : 0.99999994f) : 0.0f;
         const uint32_t q = (uint32_t)(v * 16777216.0f); /* 24 fraction bits */
@@ -259,10 +320,12 @@ void sgk_fill_eval_args(const sg_eval_plan *p, const float *coords, const int32_
     const int la = p->d >= 2 ? p->lim[p->d - 2] : 0, lb = p->lim[p->d - 1], lc = p->d >= 3 ? p->lim[p->d - 3] : 0;
     A->lim2 = p->d >= 2 ? (la < lb ? la : lb) : 0;
     A->lim3 = p->d >= 3 ? (lc < A->lim2 ? lc : A->lim2) : 0;
-    A->nparts = 1;
-    for (int k = 0; k <= SG_EVAL_MAX_PARTS; ++k) A->split[k] = k ? 0xFFFFFFFFu : 0u;
-    A->part_out = NULL;
-    A->walk = NULL;
+    A->nseg = p->seg ? p->nseg : 1;
+    A->nparts = p->seg ? p->nparts : 1;
+    A->seg = p->seg;
+    A->nshare = p->nshare > 1 && p->seg ? p->nshare : 1;
+    A->emit = A->nshare > 1 ? p->emit : SG_EMIT_SUM;
+    A->part_out = A->nshare > 1 ? p->part_out : NULL;
 }
 
 int sgk_eval_setup(void)
@@ -275,7 +338,10 @@ int sgk_eval_setup(void)
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
 #define SG_D(DD) \
-    if ((e = eval_setup<DD>()) != cudaSuccess) return e;
+    if ((e = eval_launch<DD>(nullptr, nullptr)) != cudaSuccess ||                     \
+        (e = eval_batch_launch<DD>(nullptr, nullptr, 0, nullptr)) != cudaSuccess ||   \
+        (e = eval_shared_launch<DD>(nullptr, nullptr, 0, nullptr, nullptr)) != cudaSuccess) \
+        return e;
     SG_D(1) SG_D(2) SG_D(3) SG_D(4) SG_D(5) SG_D(6) SG_D(7) SG_D(8) SG_D(9) SG_D(10)
     SG_D(11) SG_D(12) SG_D(13) SG_D(14) SG_D(15) SG_D(16) SG_D(17) SG_D(18) SG_D(19) SG_D(20)
 #undef SG_D
@@ -289,10 +355,9 @@ int sgk_evaluate(const sg_eval_plan *p, const float *coords, const int32_t *perm
     if (num_evals <= 0) return cudaSuccess;
     EvalArgs A;
     sgk_fill_eval_args(p, coords, perm, out, num_evals, &A);
-    const int ppt = p->ppt, bl = p->blocking >= 0 && p->blocking < SG_EVAL_BLOCKINGS ? p->blocking : 0;
     switch (p->d) {
 #define SG_D(DD) \
-    case DD: return eval_launch<DD>(A, ppt, bl, stream);
+    case DD: return A.nshare > 1 ? eval_shared_launch<DD>(nullptr, nullptr, 0, &A, stream) : eval_launch<DD>(&A, stream);
         SG_D(1) SG_D(2) SG_D(3) SG_D(4) SG_D(5) SG_D(6) SG_D(7) SG_D(8) SG_D(9) SG_D(10)
         SG_D(11) SG_D(12) SG_D(13) SG_D(14) SG_D(15) SG_D(16) SG_D(17) SG_D(18) SG_D(19)
         SG_D(20)
@@ -301,14 +366,14 @@ int sgk_evaluate(const sg_eval_plan *p, const float *coords, const int32_t *perm
     }
 }
 
-int sgk_evaluate_batch(int d, const sg_eval_args *grids, const int32_t *items, int nitems, int ppt, int blocking,
-                       void *stream)
+int sgk_evaluate_batch(int d, const sg_eval_args *grids, const int32_t *items, int nitems, int shared, void *stream)
 {
     const int2 *it = reinterpret_cast<const int2 *>(items);
-    const int bl = blocking >= 0 && blocking < SG_EVAL_BLOCKINGS ? blocking : 0;
     switch (d) {
 #define SG_D(DD) \
-    case DD: return eval_batch_launch<DD>(grids, it, nitems, ppt, bl, stream);
+    case DD:                                                                              \
+        return shared ? eval_shared_launch<DD>(grids, it, nitems, nullptr, stream)        \
+                      : eval_batch_launch<DD>(grids, it, nitems, stream);
         SG_D(1) SG_D(2) SG_D(3) SG_D(4) SG_D(5) SG_D(6) SG_D(7) SG_D(8) SG_D(9) SG_D(10)
         SG_D(11) SG_D(12) SG_D(13) SG_D(14) SG_D(15) SG_D(16) SG_D(17) SG_D(18) SG_D(19)
         SG_D(20)
@@ -325,12 +390,25 @@ int sgk_combine_parts(const sg_eval_args *grids, const int32_t *items, int nitem
     return cudaGetLastError();
 }
 
-int sgk_repack(const float *src, float *dst, const sg_repack *rp, int64_t nsub, void *stream)
+int sgk_combine_one(const sg_eval_plan *p, const int32_t *perm, float *out, int64_t num_evals, void *stream)
 {
-    if (nsub <= 0) return cudaSuccess;
-    int64_t g = (nsub + 7) / 8;
+    if (num_evals <= 0) return cudaSuccess;
+    k_combine_one<<<(unsigned)((num_evals + 63) / 64), 64, 0, (cudaStream_t)stream>>>(p->part_out, perm, out, num_evals,
+                                                                                    p->nseg, p->nparts, p->emit);
+    sgk_count(1);
+    return cudaGetLastError();
+}
+
+int sgk_repack(const float *src, float *dst, const sg_repack *rows, const uint32_t *offs, int64_t nrows, int n,
+               void *stream)
+{
+    if (nrows <= 0) return cudaSuccess;
+    /* a row has at most 2^n outputs (2^(s+L+1), s + L <= n-1) */
+    const int pieces = (1 << n) > kRepackPiece ? (1 << n) / kRepackPiece : 1;
+    const int64_t items = nrows * pieces;
+    int64_t g = (items + 7) / 8;
     if (g > 148 * 16) g = 148 * 16;
-    k_repack<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(src, dst, rp, nsub);
+    k_repack<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(src, dst, rows, offs, items, pieces);
     sgk_count(1);
     return cudaGetLastError();
 }

@@ -20,7 +20,7 @@ struct sg_batch {
     int64_t *doff;       /* offsets in the device value buffer (32-aligned), ng+1  */
     int64_t *boff;       /* offsets in the block-layout buffer, ng+1               */
     int dev, has_values, eval_dirty;
-    int precision, ppt, use_graph;
+    int precision, use_graph;
     int hier_kernel[SG_SWEEP_CLASSES]; /* per chain size class: 0/1 chains (where they fit), 2 gather */
     int64_t dev_bytes;
     float *d_alpha;      /* all grids, group-aligned layout                       */
@@ -51,8 +51,16 @@ struct sg_batch {
     sg_chain *d_chB[SG_MAX_DIMS];
     uint32_t *d_segB[SG_MAX_DIMS];
     /* evaluation */
-    sg_repack *d_repack;
+    sg_repack *d_repack;             /* rows of all grids                           */
+    uint32_t *d_rsrc;                /* device offsets of the rows' subspaces       */
     int64_t nrepack;
+    int max_n;                       /* largest level count among the grids         */
+    int64_t *seg_off;                /* per grid: first word of its segment table, -1: none */
+    uint32_t *d_seg;                 /* segment tables (sg_layout.h)                */
+    float *d_part;                   /* parts or segments of shared sums            */
+    int64_t part_floats;
+    int32_t *d_citems;               /* combine CTAs of the shared sums             */
+    int ncitems;
     sg_eval_args *h_eval_args, *d_eval_args;
     int32_t *h_items, *d_items;
     int64_t items_cap;
@@ -69,11 +77,7 @@ struct sg_batch {
     void *d_sscratch;                /* sort: keys, histogram, scan               */
     float *d_sorted;                 /* sorted coordinates                         */
     int32_t *d_perm;                 /* sorted position -> caller's local index    */
-    int ppt_d[SG_MAX_DIMS + 1];      /* points per thread per dimension (0: ppt) */
-    int eval_ppt_d[SG_MAX_DIMS + 1]; /* the setting the current plan was built for */
-    int blocking;                    /* SG_OPT_EVAL_BLOCKING (0: auto = wide)       */
-    int blk_d[SG_MAX_DIMS + 1];      /* tuned blocking per dimension (0: blocking) */
-    int eval_blk_d[SG_MAX_DIMS + 1]; /* the setting the current plan was built for */
+    int items_shared[SG_MAX_DIMS + 1]; /* the launch has shared sums */
     int *order;                      /* grids by dimension, most subspaces first */
     /* the per-dimension launches of an evaluation fork onto their own
      * streams (joined back before the caller's stream continues) */

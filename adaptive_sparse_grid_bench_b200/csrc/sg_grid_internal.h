@@ -26,8 +26,9 @@ struct sg_grid {
     int64_t opt[NOPT];
     float *d_alpha;   /* Npad floats, group-aligned layout         */
     double *d_work;   /* Npad doubles, FP64 hierarchization (lazy) */
-    float *d_blk;        /* N floats: surpluses in the block layout    */
-    sg_repack *d_repack; /* per-subspace compact -> block descriptors  */
+    float *d_blk;        /* Nblk floats: the block layout               */
+    sg_repack *d_repack; /* per-row compact -> block descriptors       */
+    uint32_t *d_rsrc;    /* device offsets of the rows' subspaces      */
     uint32_t blk3[SG_MAX_LEVELS]; /* block size per level budget        */
     uint32_t blk2[SG_MAX_LEVELS]; /* sub-block size per level budget    */
     int eval_dirty;      /* d_blk is stale                              */
@@ -42,9 +43,7 @@ struct sg_grid {
     int64_t dev_bytes;
     cudaEvent_t ev[SG_NUM_PHASES][2]; /* profiling: start/stop per phase */
     int ev_used[SG_NUM_PHASES];
-    uint32_t *d_walk;    /* evaluation walk tables (split sums only)     */
-    int nparts;          /* parts of a split sum in batched launches (0/1: whole) */
-    uint32_t split[SG_EVAL_MAX_PARTS + 1];
+    uint32_t *d_sums;    /* segment table of the sums (sg_layout.h), NULL: one segment */
     sg_dev_alloc_fn alloc; /* NULL: cudaMalloc/cudaFree */
     sg_dev_free_fn free_fn;
     void *alloc_ctx;
@@ -57,12 +56,8 @@ int sg_create_with_allocator(int d, int n, const int *limits, sg_dev_alloc_fn al
 
 /* Builds the block layout if the values changed since it was last built. */
 int sg_grid_prepare_eval(sg_grid *g, cudaStream_t st);
-/* Splits each point's sum over the subspaces into nparts block ranges of
- * about equal work for batched evaluations (d >= 4; otherwise, or for
- * nparts <= 1, whole sums).  Uploads the walk tables on st. */
-int sg_grid_set_parts(sg_grid *g, int nparts, cudaStream_t st);
-/* Kernel arguments to evaluate grid g at m points (device pointers); a
- * split grid's arguments carry its parts, part_out is left to the caller. */
+/* Kernel arguments to evaluate grid g at m points (device pointers),
+ * whole sums; a caller that shares them among CTAs sets nshare, emit, part_out. */
 void sg_grid_eval_args(const sg_grid *g, const float *coords, float *out, int64_t m, sg_eval_args *a);
 
 #endif

@@ -66,22 +66,28 @@ typedef struct sg_eval_plan {
     int lim[SG_MAX_DIMS];
     uint32_t blk3[SG_MAX_LEVELS]; /* block size for each level budget R      */
     uint32_t blk2[SG_MAX_LEVELS]; /* sub-block size for each level budget r  */
-    int ppt;                     /* points per thread (1 or 2)               */
-    int blocking;                /* subspace blocking preset, 0 .. SG_EVAL_BLOCKINGS-1
-                                    (wide, medium)                            */
+    int nseg, nparts;            /* segments and parts of a sum (sg_layout.h) */
+    const uint32_t *seg;         /* device segment table, NULL if nseg = 1    */
+    int nshare, emit;            /* warps per group of points, and what they write */
+    float *part_out;
 } sg_eval_plan;
 
-/* Subspace blocking presets of the evaluation kernels (SG_OPT_EVAL_BLOCKING
- * 1..2 select preset 0..1): how much of the walk runs as fully unrolled
- * blocks of compile-time shape (separate kernel instantiations for
- * 3 <= d <= 12; other d have one form).  Every preset gives bit-identical
- * results. */
+/* Values 1..SG_EVAL_BLOCKINGS of SG_OPT_EVAL_BLOCKING are accepted; the
+ * kernels have one form. */
 #define SG_EVAL_BLOCKINGS 2
 
-/* A point's sum over the subspaces can be split into up to this many
- * parts (ranges of the walk's blocks), evaluated by separate CTAs and added
- * in part order afterwards: bounds the latency of one point on a large grid. */
+/* Points per CTA of the evaluation kernels: two per thread. */
+#define SG_EVAL_CTA_POINTS 512
+
+/* A point's sum has up to this many parts (sg_layout.h). */
 #define SG_EVAL_MAX_PARTS 8
+
+/* What a launch writes of a point's sum: all of it to out; or, when several
+ * warps share it, each its parts or segments to part_out (value k of point i
+ * at part_out[k * num_evals + i]), added afterwards by sgk_combine_*. */
+#define SG_EMIT_SUM 0
+#define SG_EMIT_PARTS 1
+#define SG_EMIT_SEGS 2
 
 /* Per-grid arguments of the evaluation kernels (also the element type of
  * the batched launch's grid table). */
@@ -98,15 +104,11 @@ typedef struct sg_eval_args {
     int lim[SG_MAX_DIMS];
     uint32_t blk3[SG_MAX_LEVELS]; /* block size per budget R         */
     uint32_t blk2[SG_MAX_LEVELS]; /* sub-block size per budget r     */
-    /* split evaluation (batched launch only; nparts 1 = whole sums):
-     * part k covers the walk's blocks [split[k], split[k+1]) and writes its
-     * sums to part_out[k * num_evals + i]; walk = per (prefix depth K,
-     * budget b) the block count and block-layout extent of the subtree
-     * (sg_layout_walk_tables), used to skip subtrees outside the range. */
-    int nparts;
-    uint32_t split[SG_EVAL_MAX_PARTS + 1];
-    float *part_out;
-    const uint32_t *walk;
+    /* segments of the sums (sg_layout_seg_table); share k of nshare covers
+     * segments [k nseg / nshare, (k+1) nseg / nshare) */
+    int nseg, nparts, nshare, emit;
+    const uint32_t *seg;     /* device segment table (nseg > 1)      */
+    float *part_out;         /* emit != SG_EMIT_SUM                  */
 } sg_eval_args;
 
 void sgk_fill_eval_args(const sg_eval_plan *p, const float *coords, const int32_t *perm, float *out,
@@ -122,21 +124,22 @@ int sgk_eval_setup(void);
 int sgk_evaluate(const sg_eval_plan *p, const float *coords, const int32_t *perm, float *out,
                  int64_t num_evals, void *stream);
 /* Many grids of dimension d in one launch: items (device, 2 ints per CTA) =
- * (index into grids | part << 29, first point); each CTA covers
- * SG_EVAL_CTA_POINTS(ppt) points of its grid (index < 2^29; part selects
- * the block range of a split sum, 0 for whole sums); blocking is the
- * preset index of the launch (0 .. SG_EVAL_BLOCKINGS-1). */
-int sgk_evaluate_batch(int d, const sg_eval_args *grids, const int32_t *items, int nitems, int ppt, int blocking,
-                       void *stream);
+ * (index into grids | share << 29, first point); each CTA covers
+ * SG_EVAL_CTA_POINTS points of its grid (index < 2^29; share < the
+ * grid's nshare <= 8 selects the segments); shared: some grid has nshare > 1. */
+int sgk_evaluate_batch(int d, const sg_eval_args *grids, const int32_t *items, int nitems, int shared, void *stream);
 
-/* out[i] = compensated sum over k < nparts of part_out[k * num_evals + i]
- * (part order) for the split grids: items as for sgk_evaluate_batch, one
- * CTA per 256 points. */
+/* Adds the parts or segments in part_out to out for the grids with emit !=
+ * SG_EMIT_SUM: items as for sgk_evaluate_batch, one CTA per 256 points; or of
+ * one grid. */
 int sgk_combine_parts(const sg_eval_args *grids, const int32_t *items, int nitems, void *stream);
+int sgk_combine_one(const sg_eval_plan *p, const int32_t *perm, float *out, int64_t num_evals, void *stream);
 
-/* Reorders the surpluses from the group-aligned compact layout into the
- * block layout (one descriptor per subspace). */
-int sgk_repack(const float *src, float *dst, const sg_repack *rp, int64_t nsub, void *stream);
+/* Builds the block layout from the surpluses in the group-aligned compact
+ * layout: one descriptor per row, the device offsets of the rows' subspaces,
+ * n = the largest level count among the grids. */
+int sgk_repack(const float *src, float *dst, const sg_repack *rows, const uint32_t *offs, int64_t nrows, int n,
+               void *stream);
 
 /* Whole-grid hierarchization in shared memory for small grids, one CTA per
  * grid (all d sweeps between one load and one store). */

@@ -48,6 +48,8 @@ int sg_layout_init(sg_layout *L, int d, int n, const int *limits)
     /* kernels index the device grid with 32-bit offsets */
     if (L->Npad >= ((int64_t)1 << 31)) return SG_ERR_RANGE;
     L->Nblk = block_layout_size(L);
+    L->nrows = 0;
+    for (s = 0; s < n; s++) L->nrows += d >= 2 ? L->dp[d - 2][s] : s == 0;
     if (L->Nblk >= ((int64_t)1 << 32) - 64) return SG_ERR_RANGE;
     return SG_OK;
 }
@@ -229,8 +231,7 @@ void sg_layout_eval_sub(const sg_layout *L, int r, sg_eval_sub *sh)
         int rl = r - a < limB ? r - a : limB;
         sh->rowlen[a] = rl + 1;
         sh->aoff[a] = off;
-        /* 2^a poles of 2^rl paths of rl+1 slots */
-        off += ((uint32_t)1 << a) * (((uint32_t)1 << rl) * (uint32_t)SG_PATH_WIDTH(rl + 1));
+        off += SG_POLE_SLOTS(rl) << a; /* 2^a poles */
     }
     sh->aoff[sh->amax + 1] = off;
 }
@@ -274,48 +275,59 @@ static int64_t block_layout_size(const sg_layout *L)
     return sz[0][L->n - 1];
 }
 
-int sg_layout_eval_tables(const sg_layout *L, sg_repack **repack, uint32_t *blk3, uint32_t *blk2)
+int sg_layout_eval_tables(const sg_layout *L, sg_repack **repack, uint32_t **src, uint32_t *blk3, uint32_t *blk2)
 {
     const int d = L->d;
     const int np_dims = d >= 3 ? d - 3 : 0; /* dims 0..d-4 form the prefix */
-    int lv[SG_MAX_DIMS], k, s, R;
-    int64_t pos, r = 0;
-    /* cnt[k][R]: level vectors over prefix dims k..np_dims-1 with sum <= R;
-     * sz[k][R]: total block-layout size of their blocks (all cells) */
-    int64_t cnt[SG_MAX_DIMS + 1][SG_MAX_LEVELS], sz[SG_MAX_DIMS + 1][SG_MAX_LEVELS];
+    int lv[SG_MAX_DIMS], k, s, R, b;
+    int64_t pos, r = 0, q = 0;
+    /* sz[k][R]: total block-layout size of the blocks (all cells) of the
+     * level vectors over prefix dims k..np_dims-1 with sum <= R */
+    int64_t sz[SG_MAX_DIMS + 1][SG_MAX_LEVELS];
+    sg_eval_shape shape[SG_MAX_LEVELS];
+    sg_eval_sub subs[SG_MAX_LEVELS];
     sg_repack *rp;
+    uint32_t *so;
     for (R = 0; R < L->n; R++) {
-        sg_eval_shape sh;
-        sg_eval_sub sub;
-        sg_layout_eval_shape(L, R, &sh);
-        sg_layout_eval_sub(L, R, &sub);
-        blk3[R] = sh.coff[sh.cmax + 1];
-        blk2[R] = sub.aoff[sub.amax + 1];
-        cnt[np_dims][R] = 1;
+        sg_layout_eval_shape(L, R, &shape[R]);
+        sg_layout_eval_sub(L, R, &subs[R]);
+        blk3[R] = shape[R].coff[shape[R].cmax + 1];
+        blk2[R] = subs[R].aoff[subs[R].amax + 1];
         sz[np_dims][R] = blk3[R];
     }
     for (k = np_dims - 1; k >= 0; k--)
         for (R = 0; R < L->n; R++) {
             int l;
-            int64_t v = 0, w = 0;
-            for (l = 0; l <= R && l <= L->lim[k]; l++) {
-                v += cnt[k + 1][R - l];
-                w += sz[k + 1][R - l] << l; /* 2^l cells of this dim */
-            }
-            cnt[k][R] = v;
+            int64_t w = 0;
+            for (l = 0; l <= R && l <= L->lim[k]; l++) w += sz[k + 1][R - l] << l; /* 2^l cells of this dim */
             sz[k][R] = w;
         }
     if (sz[0][L->n - 1] != L->Nblk) return SG_ERR_STATE;
-    rp = (sg_repack *)malloc((size_t)(L->S > 0 ? L->S : 1) * sizeof(sg_repack));
-    if (!rp) return SG_ERR_NOMEM;
+    rp = (sg_repack *)malloc((size_t)L->nrows * sizeof(sg_repack));
+    so = (uint32_t *)malloc((size_t)L->S * sizeof(uint32_t));
+    if (!rp || !so) {
+        free(rp);
+        free(so);
+        return SG_ERR_NOMEM;
+    }
     memset(lv, 0, sizeof(lv));
-    for (s = 0; s < L->n; s++)
-        for (pos = 0; pos < L->dp[d - 1][s]; pos++) {
-            int c, a, b, rem = L->n - 1, sigma = 0;
-            int64_t base = 0, scale = 1;
-            sg_eval_shape sh;
-            sg_eval_sub sub;
-            sg_layout_idx2l(L, pos, s, lv);
+    for (s = 0; s < L->n; s++) {
+        /* the level vectors of dims 0..d-2 with sum s, in the order of the
+         * (d-1)-dimensional positions */
+        const int64_t cnt = d >= 2 ? L->dp[d - 2][s] : s == 0;
+        const int last = L->n - 1 - s < L->lim[d - 1] ? L->n - 1 - s : L->lim[d - 1];
+        for (pos = 0; pos < cnt; pos++) {
+            int c, a, rem = L->n - 1, sigma = 0, rest = s;
+            int64_t base = 0, scale = 1, p = pos;
+            const sg_eval_shape *sh;
+            const sg_eval_sub *sub;
+            for (k = d - 2; k >= 1; k--) {
+                int level = 0;
+                while (p >= L->dp[k - 1][rest - level]) p -= L->dp[k - 1][rest - level++];
+                lv[k] = level;
+                rest -= level;
+            }
+            if (d >= 2) lv[0] = rest;
             /* block-layout start of this prefix: the sizes of all prefixes
              * that precede it in the depth-first walk */
             for (k = 0; k < np_dims; k++) {
@@ -327,117 +339,125 @@ int sg_layout_eval_tables(const sg_layout *L, sg_repack **repack, uint32_t *blk3
             }
             c = d >= 3 ? lv[d - 3] : 0;
             a = d >= 2 ? lv[d - 2] : 0;
-            b = lv[d - 1];
-            sg_layout_eval_shape(L, L->n - 1 - sigma, &sh);
-            sg_layout_eval_sub(L, L->n - 1 - sigma - c, &sub);
-            rp[r].src = (uint32_t)(L->plidx[s] + (pos << s));
-            rp[r].dst = (uint32_t)base + sh.coff[c] + sub.aoff[a] + (uint32_t)b;
-            rp[r].blk = sh.coff[sh.cmax + 1];
-            rp[r].sub = sub.aoff[sub.amax + 1];
-            rp[r].plen = ((uint32_t)1 << (sub.rowlen[a] - 1)) * (uint32_t)SG_PATH_WIDTH(sub.rowlen[a]);
-            rp[r].L = (uint8_t)(sub.rowlen[a] - 1);
-            rp[r].pad[0] = rp[r].pad[1] = rp[r].pad[2] = 0;
+            sh = &shape[L->n - 1 - sigma];
+            sub = &subs[L->n - 1 - sigma - c];
+            rp[r].src = (uint32_t)q;
+            rp[r].dst = (uint32_t)base + sh->coff[c] + sub->aoff[a];
+            rp[r].blk = sh->coff[sh->cmax + 1];
+            rp[r].sub = sub->aoff[sub->amax + 1];
+            rp[r].plen = SG_POLE_SLOTS(last);
             rp[r].c = (uint8_t)c;
             rp[r].a = (uint8_t)a;
-            rp[r].b = (uint8_t)b;
+            rp[r].L = (uint8_t)last;
             rp[r].s = (uint8_t)s;
             r++;
-        }
-    *repack = rp;
-    return SG_OK;
-}
-
-/* ---- walk tables and split evaluation ----------------------------------- */
-
-int sg_layout_walk_tables(const sg_layout *L, const uint32_t *blk3, uint32_t *walk)
-{
-    const int d = L->d, n = L->n;
-    int K, b, l;
-    if (d < 4) return SG_ERR_ARG;
-    for (b = 0; b < n; b++) {
-        walk[2 * ((d - 3) * n + b)] = 1;
-        walk[2 * ((d - 3) * n + b) + 1] = blk3[b] << (n - 1 - b);
-    }
-    for (K = d - 4; K >= 0; K--)
-        for (b = 0; b < n; b++) {
-            uint64_t cnt = 0, ext = 0;
-            for (l = 0; l <= b && l <= L->lim[K]; l++) {
-                cnt += walk[2 * ((K + 1) * n + b - l)];
-                ext += walk[2 * ((K + 1) * n + b - l) + 1];
+            /* subspace (lv, b): its position adds the vectors with a lower
+             * level of dim d-1 */
+            for (b = 0; b <= last; b++) {
+                int64_t at = pos;
+                int j;
+                for (j = 0; d >= 2 && j < b; j++) at += L->dp[d - 2][s + b - j];
+                so[q++] = (uint32_t)(L->plidx[s + b] + (at << (s + b)));
             }
-            walk[2 * (K * n + b)] = (uint32_t)cnt;
-            walk[2 * (K * n + b) + 1] = (uint32_t)ext;
         }
+    }
+    if (r != L->nrows || q != L->S) {
+        free(rp);
+        free(so);
+        return SG_ERR_STATE;
+    }
+    *repack = rp;
+    *src = so;
     return SG_OK;
 }
 
-/* subspaces (c, a, b) of the innermost dims with c + a + b <= R, in limits */
-static double block_subspaces(const sg_layout *L, int R)
+/* ---- segments of the evaluation's sums ---------------------------------- */
+
+int sg_layout_parts(const sg_layout *L)
 {
-    const int lc = L->lim[L->d - 3], la = L->lim[L->d - 2], lb = L->lim[L->d - 1];
+    if (L->d < 4 || L->S < 4096) return 1;
+    return L->S / 2048 < 8 ? (int)(L->S / 2048) : 8;
+}
+
+int sg_layout_segs(const sg_layout *L)
+{
+    const int parts = sg_layout_parts(L);
+    if (L->d < 4) return 1;
+    if (parts > 1) return parts * SG_SEG_PER_PART;
+    if (L->S < 2 * SG_SEG_SUBSPACES) return 1;
+    return L->S / SG_SEG_SUBSPACES < SG_SEG_PER_PART ? (int)(L->S / SG_SEG_SUBSPACES) : SG_SEG_PER_PART;
+}
+
+int64_t sg_layout_seg_words(const sg_layout *L)
+{
+    const int nseg = sg_layout_segs(L);
+    return nseg > 1 ? (int64_t)(L->d - 2) * L->n + nseg + 1 : 0;
+}
+
+/* rows (c, a) of the innermost dims with c + a <= R, in limits */
+static double block_rows(const sg_layout *L, int R)
+{
+    const int lc = L->lim[L->d - 3], la = L->lim[L->d - 2];
     double cnt = 0.0;
-    int c, a;
-    for (c = 0; c <= R && c <= lc; c++)
-        for (a = 0; a <= R - c && a <= la; a++) cnt += (R - c - a < lb ? R - c - a : lb) + 1;
+    int c;
+    for (c = 0; c <= R && c <= lc; c++) cnt += (R - c < la ? R - c : la) + 1;
     return cnt;
 }
 
-#define SG_BLOCK_OVERHEAD 3.0 /* per-block walk cost in subspace-equivalents */
+#define SG_BLOCK_OVERHEAD 2.0 /* per-block walk cost in rows */
 
-int sg_layout_walk_split(const sg_layout *L, int nparts, uint32_t *bounds)
+int sg_layout_seg_table(const sg_layout *L, const uint32_t *blk3, uint32_t *table)
 {
-    const int d = L->d, n = L->n;
+    const int d = L->d, n = L->n, nseg = sg_layout_segs(L);
+    /* deepest loop whose iterations a segment may start at: the dims from
+     * d-4 on run as one unit (d = 4: its only loop) */
+    const int deep = d == 4 ? 0 : d - 5;
+    uint32_t *bounds = table + (d - 2) * n;
     double *W;
-    uint32_t *cnt;
     int K, b, l, j;
-    if (d < 4 || nparts < 1) return SG_ERR_ARG;
+    if (nseg <= 1) return SG_ERR_ARG;
     W = (double *)malloc(sizeof(double) * (size_t)(d - 2) * (size_t)n);
-    cnt = (uint32_t *)malloc(sizeof(uint32_t) * (size_t)(d - 2) * (size_t)n);
-    if (!W || !cnt) {
-        free(W);
-        free(cnt);
-        return SG_ERR_NOMEM;
-    }
+    if (!W) return SG_ERR_NOMEM;
     for (b = 0; b < n; b++) {
-        W[(d - 3) * n + b] = block_subspaces(L, b) + SG_BLOCK_OVERHEAD;
-        cnt[(d - 3) * n + b] = 1;
+        W[(d - 3) * n + b] = block_rows(L, b) + SG_BLOCK_OVERHEAD;
+        table[(d - 3) * n + b] = blk3[b] << (n - 1 - b);
     }
     for (K = d - 4; K >= 0; K--)
         for (b = 0; b < n; b++) {
             double w = 0.0;
-            uint64_t c = 0;
+            uint64_t ext = 0;
             for (l = 0; l <= b && l <= L->lim[K]; l++) {
                 w += W[(K + 1) * n + b - l];
-                c += cnt[(K + 1) * n + b - l];
+                ext += table[(K + 1) * n + b - l];
             }
             W[K * n + b] = w;
-            cnt[K * n + b] = (uint32_t)c;
+            table[K * n + b] = (uint32_t)ext;
         }
     bounds[0] = 0;
-    bounds[nparts] = cnt[n - 1];
-    for (j = 1; j < nparts; j++) {
-        /* descend to the block holding work position j/nparts of the total */
-        const double t = W[n - 1] * j / nparts;
+    bounds[nseg] = table[n - 1];
+    for (j = 1; j < nseg; j++) {
+        /* descend to the unit holding work position j/nseg of the total; the
+         * segment starts where the unit does.  Units: iterations of the loop
+         * at depth `deep`, and whole nodes of that depth with a budget the
+         * kernels may unroll (SG_SEG_UNIT_BUDGET) */
+        const double t = W[n - 1] * j / nseg;
         double acc = 0.0;
-        uint32_t leaf = 0;
+        uint32_t at = 0;
         K = 0;
         b = n - 1;
-        while (K < d - 3) {
+        while (K <= deep && !(K == deep && d > 4 && b <= SG_SEG_UNIT_BUDGET)) {
             const int lmax = b < L->lim[K] ? b : L->lim[K];
-            for (l = 0; l <= lmax; l++) {
+            for (l = 0; l < lmax; l++) {
                 const double w = W[(K + 1) * n + b - l];
                 if (acc + w > t) break;
                 acc += w;
-                leaf += cnt[(K + 1) * n + b - l];
+                at += table[(K + 1) * n + b - l];
             }
-            if (l > lmax) break; /* rounding: t at the very end */
             K++;
             b -= l;
         }
-        bounds[j] = leaf < bounds[j - 1] ? bounds[j - 1] : leaf;
-        if (bounds[j] > bounds[nparts]) bounds[j] = bounds[nparts];
+        bounds[j] = at < bounds[j - 1] ? bounds[j - 1] : at;
     }
     free(W);
-    free(cnt);
     return SG_OK;
 }

@@ -30,7 +30,8 @@ typedef struct sg_layout {
     int64_t lidx[SG_MAX_LEVELS + 1];        /* compact group offsets        */
     int64_t plidx[SG_MAX_LEVELS + 1];       /* device (padded) group offsets */
     int64_t N, S, Npad;
-    int64_t Nblk; /* values of the evaluation (block) layout */
+    int64_t Nblk;  /* slots of the evaluation (block) layout             */
+    int64_t nrows; /* rows of dim B in it (level vectors of dims 0..d-2) */
 } sg_layout;
 
 /* One 1-D "chain" of sweep k: the subspaces that differ only in l_k.  They
@@ -69,20 +70,23 @@ int sg_layout_chains(const sg_layout *L, int k, sg_chain **chains, int64_t *ncha
  *   planes c = 0..cmax, each 2^c sub-blocks (one per cell t_c of dim C);
  *   a sub-block of budget r = R-c has rows a = 0..amax(r), each 2^a poles
  *   (one per cell t_a of dim A);
- *   a pole holds dim B's levels b = 0..L (L = rowlen-1) as 2^L paths, one
- *   per finest cell t_L: path t_L is the L+1 surpluses a query point in that
- *   cell needs, level b's cell t_L >> (L-b) in slot b, in W = L+1 rounded up
- *   to even slots (SG_PATH_WIDTH).  A surplus of level b therefore appears
- *   in 2^(L-b) paths (Nblk >= N values in all).
- * A query point finds the surplus of (c, a, b) at
- *   base + coff(c) + t_c * sub(R-c) + aoff(R-c, a) + t_a * plen + t_L * W + b,
- * so the loads of a row share one address and differ by a constant; every
- * row with L >= 1 starts at an even offset (all sizes before it in a block
- * are even), so slots 2j, 2j+1 move with one 8-byte load.
+ *   a pole holds what a query point needs of dim B's levels b = 0..L (L =
+ *   rowlen-1), in one slot or one 8-byte pair per point:
+ *     L = 0: the one surplus;
+ *     L = 1: per cell t of level 1 the pair (surplus of level 0, surplus of
+ *       level 1 in cell t);
+ *     L >= 2: the levels summed.  The sum over b of surplus * hat is linear
+ *       in x_B on each of the 2^(L+1) halves of the cells of level L; half h
+ *       holds the pair (value at its left end, value at its right end minus
+ *       that), both summed in FP64 from the surpluses and rounded once.
+ * A query point finds the pair of row (c, a) at
+ *   base + coff(c) + t_c * sub(R-c) + aoff(R-c, a) + t_a * plen + 2 t_B
+ * with t_B its cell of level 1 (L = 1) or its half (L >= 2).  Every row with
+ * L >= 1 starts at an even offset (all sizes before it in a block are even),
+ * so a pair moves with one 8-byte load.
  */
-/* Slots of a path of `levels` levels: rounded up to an even count (two
- * levels per 8-byte load), a single level alone. */
-#define SG_PATH_WIDTH(levels) ((levels) <= 1 ? (levels) : (((levels) + 1) & ~1))
+/* Slots of a pole whose last level of dim B is L. */
+#define SG_POLE_SLOTS(L) ((L) == 0 ? 1u : ((L) == 1 ? 4u : 4u << (L)))
 
 typedef struct sg_eval_sub {
     int amax;                         /* last row: min(r, lim_A)           */
@@ -98,31 +102,46 @@ typedef struct sg_eval_shape {
 void sg_layout_eval_sub(const sg_layout *L, int r, sg_eval_sub *sh);
 void sg_layout_eval_shape(const sg_layout *L, int R, sg_eval_shape *sh);
 
-/* Walk tables of the evaluation (d >= 4; the walk visits prefix dims
- * 0..d-4, blocks sit at depth d-3).  For depth K = 0..d-3 and budget
- * b = 0..n-1: walk[2*(K*n + b)] = number of blocks of the subtree entered at
- * depth K with budget b, walk[2*(K*n + b) + 1] = their extent in the block
- * layout (sum of blk3[R] << (n-1-R)).  walk has 2*(d-2)*n entries. */
-int sg_layout_walk_tables(const sg_layout *L, const uint32_t *blk3, uint32_t *walk);
-/* bounds[0..nparts]: block ranges of the walk with about equal work each
- * (subspaces per block plus a per-block overhead); d >= 4. */
-int sg_layout_walk_split(const sg_layout *L, int nparts, uint32_t *bounds);
+/* Segments of a point's sum.  The evaluation adds up a point's sum in
+ * segments of consecutive blocks of the walk, each with its own compensated
+ * sum, the segments of a part (SG_SEG_PER_PART of them) into the part's and the
+ * parts into the total.  The bounds depend on the grid alone, so one thread
+ * adding everything and many warps adding a few segments each give the same
+ * bits.  nseg = 1 for small grids and d < 4; parts = 1 or nseg / SG_SEG_PER_PART.
+ * A warp's chain of dependent work is then S / nseg subspaces at the shortest:
+ * about 128 of them, below which a segment's walk down from the root costs as
+ * much as its sums. */
+#define SG_SEG_PER_PART 16
+#define SG_SEG_SUBSPACES 128
+#define SG_MAX_SEGS (SG_SEG_PER_PART * 8)
+#define SG_SEG_UNIT_BUDGET 3 /* the kernels' SG_EVAL_MAX_LEAF2 */
+int sg_layout_parts(const sg_layout *L);
+int sg_layout_segs(const sg_layout *L);
+/* Words of the segment table: the extents in the block layout of the subtree
+ * of the walk entered at depth K = 0..d-3 with budget b = 0..n-1, at K*n + b
+ * (the walk visits prefix dims 0..d-4, blocks sit at depth d-3), then the
+ * nseg+1 bounds as block-layout offsets.  0 when nseg = 1. */
+int64_t sg_layout_seg_words(const sg_layout *L);
+int sg_layout_seg_table(const sg_layout *L, const uint32_t *blk3, uint32_t *table);
 
-/* Per-subspace repack descriptor (compact layout -> block layout). */
+/* Per-row repack descriptor (compact layout -> block layout): the row of
+ * one level vector of dims 0..d-2, whose levels 0..L of dim B are L+1
+ * subspaces. */
 typedef struct sg_repack {
-    uint32_t src;  /* device offset of the subspace in the group-aligned layout */
-    uint32_t dst;  /* block-layout offset of its element with I = t = 0 (slot b) */
+    uint32_t src;  /* first of its L+1 entries in the table of subspace offsets */
+    uint32_t dst;  /* block-layout offset of its first slot with I = t = 0      */
     uint32_t blk;  /* block size: stride of the prefix cell I                   */
     uint32_t sub;  /* sub-block size: stride of t_c                             */
-    uint32_t plen; /* pole length: stride of t_a                                */
-    uint8_t c, a, b, s;
-    uint8_t L;     /* last level of dim B in the row: paths of L+1 slots        */
-    uint8_t pad[3];
+    uint32_t plen; /* pole size: stride of t_a                                  */
+    uint8_t c, a;  /* levels of dims C and A                                    */
+    uint8_t L;     /* last level of dim B                                       */
+    uint8_t s;     /* level sum of dims 0..d-2: 2^s poles                       */
 } sg_repack;
 
-/* The repack table (one entry per subspace, malloc'd) and the block sizes
- * blk3[R] (3-D block) and blk2[r] (sub-block) for every budget. */
-int sg_layout_eval_tables(const sg_layout *L, sg_repack **repack, uint32_t *blk3, uint32_t *blk2);
+/* The repack table (nrows entries), the device offsets of the rows'
+ * subspaces (S entries; both malloc'd) and the block sizes blk3[R] (3-D
+ * block) and blk2[r] (sub-block) for every budget. */
+int sg_layout_eval_tables(const sg_layout *L, sg_repack **repack, uint32_t **src, uint32_t *blk3, uint32_t *blk2);
 
 #ifdef __cplusplus
 }

@@ -93,6 +93,7 @@ static void free_device(sg_grid *g)
     dev_free(g, g->d_work);
     dev_free(g, g->d_blk);
     dev_free(g, g->d_repack);
+    dev_free(g, g->d_rsrc);
     for (k = 0; k < SG_MAX_DIMS; k++) {
         dev_free(g, g->d_chains[k]);
         dev_free(g, g->d_seg[k]);
@@ -100,7 +101,7 @@ static void free_device(sg_grid *g)
     dev_free(g, g->d_err);
     dev_free(g, g->d_scratch);
     dev_free(g, g->d_io);
-    dev_free(g, g->d_walk);
+    dev_free(g, g->d_sums);
 }
 
 int sg_create_with_allocator(int d, int n, const int *limits, sg_dev_alloc_fn alloc, sg_dev_free_fn free_fn,
@@ -258,6 +259,8 @@ static int materialize(sg_grid *g, cudaStream_t st)
 {
     const sg_layout *L = &g->L;
     sg_repack *rp = NULL;
+    uint32_t *rs = NULL, *st_tab = NULL;
+    int64_t words;
     int k, r;
     cudaError_t ce;
     if (g->dev >= 0) return SG_OK;
@@ -273,21 +276,39 @@ static int materialize(sg_grid *g, cudaStream_t st)
         r = cuda_fail(ce, "cudaMemsetAsync");
         goto bad;
     }
-    if ((r = sg_layout_eval_tables(L, &rp, g->blk3, g->blk2)) != SG_OK) {
+    if ((r = sg_layout_eval_tables(L, &rp, &rs, g->blk3, g->blk2)) != SG_OK) {
         fail(r, "building the evaluation layout tables");
         goto bad;
     }
     if ((r = dev_alloc(g, (void **)&g->d_blk, L->Nblk * 4, "block layout")) != SG_OK) goto bad;
-    if ((r = dev_alloc(g, (void **)&g->d_repack, L->S * (int64_t)sizeof(sg_repack), "repack table")) != SG_OK)
+    if ((r = dev_alloc(g, (void **)&g->d_repack, L->nrows * (int64_t)sizeof(sg_repack), "repack table")) != SG_OK ||
+        (r = dev_alloc(g, (void **)&g->d_rsrc, L->S * 4, "repack offsets")) != SG_OK)
         goto bad;
-    /* pageable sources: the copy has taken the bytes when the call returns */
-    if ((ce = cudaMemcpyAsync(g->d_repack, rp, (size_t)L->S * sizeof(sg_repack), cudaMemcpyHostToDevice, st)) !=
-        cudaSuccess) {
+    /* pageable sources: the copies have taken the bytes when the calls return */
+    ce = cudaMemcpyAsync(g->d_repack, rp, (size_t)L->nrows * sizeof(sg_repack), cudaMemcpyHostToDevice, st);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(g->d_rsrc, rs, (size_t)L->S * 4, cudaMemcpyHostToDevice, st);
+    if (ce != cudaSuccess) {
         r = cuda_fail(ce, "uploading the repack table");
         goto bad;
     }
     free(rp);
+    free(rs);
     rp = NULL;
+    rs = NULL;
+    if ((words = sg_layout_seg_words(L)) > 0) {
+        st_tab = (uint32_t *)malloc((size_t)words * 4);
+        if (!st_tab || (r = sg_layout_seg_table(L, g->blk3, st_tab)) != SG_OK) {
+            r = fail(SG_ERR_NOMEM, "building the segment table");
+            goto bad;
+        }
+        if ((r = dev_alloc(g, (void **)&g->d_sums, words * 4, "segment table")) != SG_OK) goto bad;
+        if ((ce = cudaMemcpyAsync(g->d_sums, st_tab, (size_t)words * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
+            r = cuda_fail(ce, "uploading the segment table");
+            goto bad;
+        }
+        free(st_tab);
+        st_tab = NULL;
+    }
     g->eval_dirty = 1;
     for (k = 0; k < L->d; k++) {
         sg_chain *ch = NULL;
@@ -336,6 +357,8 @@ static int materialize(sg_grid *g, cudaStream_t st)
 bad:
     cudaStreamSynchronize(st); /* nothing may still write the ranges freed below */
     free(rp);
+    free(rs);
+    free(st_tab);
     free_device(g);
     memset(g->d_chains, 0, sizeof(g->d_chains));
     memset(g->d_seg, 0, sizeof(g->d_seg));
@@ -343,8 +366,9 @@ bad:
     g->d_work = NULL;
     g->d_blk = NULL;
     g->d_repack = NULL;
+    g->d_rsrc = NULL;
     g->d_err = NULL;
-    g->d_walk = NULL;
+    g->d_sums = NULL;
     g->d_scratch = g->d_io = NULL;
     g->scratch_bytes = g->io_bytes = g->dev_bytes = 0;
     g->dev = -1;
@@ -585,7 +609,7 @@ SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_
         g->opt[SG_OPT_EVAL_PPT] = ppts[bi / 2];
         g->opt[SG_OPT_EVAL_SORT] = bi % 2;
     }
-    /* subspace blocking at that setting (scratch and layout are built) */
+    /* under each blocking value (one kernel form: two timings of the same) */
     for (i = 0, best = 1e30, bi = -1; i < SG_EVAL_BLOCKINGS && r == SG_OK; i++) {
         g->opt[SG_OPT_EVAL_BLOCKING] = i + 1;
         r = time_best(tune_eval_once, g, &ta, ta.st, 2, &t[6 + i]);
@@ -657,15 +681,8 @@ static int ensure(sg_grid *g, void **buf, int64_t *have, int64_t need, const cha
     return SG_OK;
 }
 
-static int eval_ppt(const sg_grid *g)
-{
-    if (g->opt[SG_OPT_EVAL_PPT] == 1 || g->opt[SG_OPT_EVAL_PPT] == 2) return (int)g->opt[SG_OPT_EVAL_PPT];
-    return 2;
-}
-
-/* The evaluation plan of the grid's block layout at `ppt` points per
- * thread and the grid's blocking setting (0 = auto: wide). */
-static void grid_plan(const sg_grid *g, int ppt, sg_eval_plan *p)
+/* The evaluation plan of the grid's block layout, whole sums. */
+static void grid_plan(const sg_grid *g, sg_eval_plan *p)
 {
     int k;
     p->alpha = g->d_blk;
@@ -676,42 +693,124 @@ static void grid_plan(const sg_grid *g, int ppt, sg_eval_plan *p)
         p->blk3[k] = g->blk3[k];
         p->blk2[k] = g->blk2[k];
     }
-    p->ppt = ppt;
-    p->blocking = g->opt[SG_OPT_EVAL_BLOCKING] > 0 ? (int)g->opt[SG_OPT_EVAL_BLOCKING] - 1 : 0;
+    p->nseg = g->d_sums ? sg_layout_segs(&g->L) : 1;
+    p->nparts = g->d_sums ? sg_layout_parts(&g->L) : 1;
+    p->seg = g->d_sums;
+    p->nshare = 1;
+    p->emit = SG_EMIT_SUM;
+    p->part_out = NULL;
+}
+
+#define SG_SHARE_ROUNDS 3                  /* resident warps' worth of warps to aim for      */
+#define SG_SHARE_MIN_SEGS 4                /* fewer segments: adding them up costs more     */
+#define SG_SHARE_FLOATS ((int64_t)1 << 25) /* largest buffer of segment sums                */
+#define SG_SORT_ROWS ((int64_t)3 << 24)    /* points x rows from which ordering pays        */
+#define SG_SORT_BYTES (192 * 1024)         /* block layouts up to an L1 need no ordering    */
+
+/* How many warps share a point's sum.  A launch with few points leaves most of
+ * the GPU idle while each thread works through all S subspaces, so where the
+ * whole-sum launch would fill less than 3/4 of its rounds of resident warps (16
+ * per SM, 64 points each) the segments of a sum go to several warps.  (The
+ * kernel that can share is about a quarter slower per point than the one that
+ * cannot.)  d = 10, n = 10: 7.35 -> 0.17 ms for 1,000 points, 6.05 -> 3.3 ms for
+ * 65,536; 2^20 points share at a loss (35.3 -> 42.9 ms).  Returns the floats of
+ * part_out (0: whole sums).  No choice changes a result. */
+static int64_t plan_shares(const sg_grid *g, int64_t m, sg_eval_plan *p)
+{
+    const int64_t room = (int64_t)sgk_num_sms() * 16, groups = (m + 63) / 64;
+    int64_t want, floats;
+    /* a pool's grids take no scratch beyond the sort's */
+    if (p->nseg < SG_SHARE_MIN_SEGS || g->alloc) return 0;
+    if (4 * groups >= 3 * ((groups + room - 1) / room * room)) return 0;
+    want = (SG_SHARE_ROUNDS * room + groups - 1) / groups;
+    if (want <= p->nparts) {
+        p->nshare = p->nparts;
+        p->emit = SG_EMIT_PARTS;
+        floats = p->nparts * m;
+    } else {
+        p->nshare = want < p->nseg ? (int)want : p->nseg;
+        p->emit = SG_EMIT_SEGS;
+        floats = p->nseg * m;
+    }
+    if (floats <= SG_SHARE_FLOATS) return floats;
+    p->nshare = 1;
+    p->emit = SG_EMIT_SUM;
+    return 0;
+}
+
+/* Whether to put the points in spatial order first: it makes a warp's gathers
+ * share cache lines, at four or more launches.  Measured to pay from about
+ * 50 M points x rows on (d = 10, n = 10: 1,000 points; d = 6, n = 8: 65,536), and
+ * not at all for a layout that fits L1 (d = 4, n = 8: 2^20 points 136 us in
+ * caller order, 171 us ordered).  No choice changes a result. */
+static int plan_sort(const sg_grid *g, int64_t m)
+{
+    return g->opt[SG_OPT_EVAL_SORT] && m * g->L.nrows >= SG_SORT_ROWS && g->L.Nblk * 4 > SG_SORT_BYTES;
+}
+
+/* The evaluation launches, with scratch for the sort (sort != 0) followed by
+ * the segment sums. */
+typedef struct eval_scratch {
+    int64_t sort_b, coords_b, perm_b, part_b; /* bytes of each region */
+} eval_scratch;
+
+static int64_t scratch_plan(int64_t m, int d, int sort, int64_t part_floats, eval_scratch *s)
+{
+    s->sort_b = sort ? (sgk_sort_scratch_bytes(m, d) + 255) & ~(int64_t)255 : 0;
+    s->coords_b = sort ? (m * d * 4 + 255) & ~(int64_t)255 : 0;
+    s->perm_b = sort ? (m * 4 + 255) & ~(int64_t)255 : 0;
+    s->part_b = part_floats * 4;
+    return s->sort_b + s->coords_b + s->perm_b + s->part_b;
+}
+
+static int evaluate_with(sg_grid *g, sg_eval_plan *p, const eval_scratch *s, char *base, int profile,
+                         const float *coords, float *out, int64_t m, cudaStream_t st)
+{
+    const int32_t *perm = NULL;
+    int e;
+    if (g->eval_dirty) {
+        if ((e = sgk_repack(g->d_alpha, g->d_blk, g->d_repack, g->d_rsrc, g->L.nrows, g->L.n, st)) != cudaSuccess)
+            return cuda_fail((cudaError_t)e, "repacking surpluses");
+        g->eval_dirty = 0;
+    }
+    if (s->sort_b) {
+        float *sorted = (float *)(base + s->sort_b);
+        perm = (const int32_t *)(base + s->sort_b + s->coords_b);
+        if (profile) mark(g, SG_PHASE_SORT, 0, st);
+        /* the histogram is cleared inside the sort, so nothing left in the
+         * scratch by an earlier call is read */
+        if ((e = sgk_sort_points(coords, m, p->d, base, sorted, (int32_t *)perm, st)) != cudaSuccess)
+            return cuda_fail((cudaError_t)e, "sorting query points");
+        if (profile) mark(g, SG_PHASE_SORT, 1, st);
+        coords = sorted;
+    }
+    if (profile) mark(g, SG_PHASE_EVALUATE, 0, st);
+    p->part_out = s->part_b ? (float *)(base + s->sort_b + s->coords_b + s->perm_b) : NULL;
+    e = sgk_evaluate(p, coords, perm, out, m, st);
+    if (e == cudaSuccess && p->nshare > 1) e = sgk_combine_one(p, perm, out, m, st);
+    if (profile) mark(g, SG_PHASE_EVALUATE, 1, st);
+    return e == cudaSuccess ? SG_OK : cuda_fail((cudaError_t)e, "evaluate");
 }
 
 static int evaluate_on(sg_grid *g, const float *coords, float *out, int64_t m, cudaStream_t st)
 {
     sg_eval_plan p;
-    int e;
-    if (g->eval_dirty) {
-        if ((e = sgk_repack(g->d_alpha, g->d_blk, g->d_repack, g->L.S, st)) != cudaSuccess)
-            return cuda_fail((cudaError_t)e, "repacking surpluses");
-        g->eval_dirty = 0;
+    eval_scratch s;
+    int64_t need, parts;
+    const int sort = plan_sort(g, m);
+    int r;
+    grid_plan(g, &p);
+    parts = plan_shares(g, m, &p);
+    need = scratch_plan(m, p.d, sort, parts, &s);
+    r = need ? ensure(g, &g->d_scratch, &g->scratch_bytes, need, "evaluate scratch") : SG_OK;
+    if (r == SG_ERR_NOMEM && parts) {
+        /* no room for the segment sums: whole sums need none */
+        p.nshare = 1;
+        p.emit = SG_EMIT_SUM;
+        need = scratch_plan(m, p.d, sort, 0, &s);
+        r = need ? ensure(g, &g->d_scratch, &g->scratch_bytes, need, "evaluate scratch") : SG_OK;
     }
-    grid_plan(g, eval_ppt(g), &p);
-    if (g->opt[SG_OPT_EVAL_SORT] && m > 1) {
-        const int64_t sort_b = (sgk_sort_scratch_bytes(m, p.d) + 255) & ~(int64_t)255;
-        const int64_t coords_b = (m * p.d * 4 + 255) & ~(int64_t)255;
-        int r = ensure(g, &g->d_scratch, &g->scratch_bytes, sort_b + coords_b + m * 4, "evaluate scratch");
-        char *base = (char *)g->d_scratch;
-        float *sorted = (float *)(base + sort_b);
-        int32_t *perm = (int32_t *)(base + sort_b + coords_b);
-        if (r != SG_OK) return r;
-        mark(g, SG_PHASE_SORT, 0, st);
-        if ((e = sgk_sort_points(coords, m, p.d, base, sorted, perm, st)) != cudaSuccess)
-            return cuda_fail((cudaError_t)e, "sorting query points");
-        mark(g, SG_PHASE_SORT, 1, st);
-        mark(g, SG_PHASE_EVALUATE, 0, st);
-        e = sgk_evaluate(&p, sorted, perm, out, m, st);
-        mark(g, SG_PHASE_EVALUATE, 1, st);
-    } else {
-        mark(g, SG_PHASE_EVALUATE, 0, st);
-        e = sgk_evaluate(&p, coords, NULL, out, m, st);
-        mark(g, SG_PHASE_EVALUATE, 1, st);
-    }
-    if (e != cudaSuccess) return cuda_fail((cudaError_t)e, "evaluate");
-    return SG_OK;
+    return r == SG_OK ? evaluate_with(g, &p, &s, (char *)g->d_scratch, 1, coords, out, m, st) : r;
 }
 
 SG_API int sg_evaluate_device(sg_grid *g, const float *coords, float *out, int64_t m, void *stream)
@@ -732,11 +831,11 @@ SG_API int sg_evaluate_device(sg_grid *g, const float *coords, float *out, int64
  * device memory, event or other resource is created. */
 SG_API int sg_evaluate_device_noalloc(sg_grid *g, const float *coords, float *out, int64_t m, void *stream)
 {
-    cudaStream_t st = (cudaStream_t)stream;
     sg_eval_plan p;
-    int prev, r = SG_OK, e, k;
+    eval_scratch s;
+    int prev, r = SG_OK, e, sort;
     void *scratch = NULL;
-    int64_t have = 0, sort_b, coords_b;
+    int64_t have = 0, need, parts;
     if (!g || m < 0 || (m > 0 && (!coords || !out))) return fail(SG_ERR_ARG, "sg_evaluate_device_noalloc: bad argument");
     if (!g->has_values || g->dev < 0)
         return fail(SG_ERR_STATE, "sg_evaluate_device_noalloc: the grid has no device state yet (set values first)");
@@ -744,33 +843,25 @@ SG_API int sg_evaluate_device_noalloc(sg_grid *g, const float *coords, float *ou
         return fail(SG_ERR_RANGE, "sg_evaluate_device_noalloc: %lld points exceed SG_NOALLOC_MAX_POINTS (%d)",
                     (long long)m, SG_NOALLOC_MAX_POINTS);
     if (m == 0) return SG_OK;
-    sort_b = (sgk_sort_scratch_bytes(m, g->L.d) + 255) & ~(int64_t)255;
-    coords_b = (m * g->L.d * 4 + 255) & ~(int64_t)255;
     if ((r = enter(g, &prev)) != SG_OK) return r;
+    grid_plan(g, &p);
+    parts = plan_shares(g, m, &p);
+    sort = plan_sort(g, m);
+    need = scratch_plan(m, g->L.d, sort, parts, &s);
     if ((e = sgk_noalloc_scratch(&scratch, &have)) != cudaSuccess) {
         r = cuda_fail((cudaError_t)e, "sg_evaluate_device_noalloc: scratch address");
-    } else if (sort_b + coords_b + m * 4 > have) {
-        r = fail(SG_ERR_RANGE, "sg_evaluate_device_noalloc: %lld points in %d dims need more than the %lld-byte scratch",
-                 (long long)m, g->L.d, (long long)have);
     } else {
-        char *base = (char *)scratch;
-        float *sorted = (float *)(base + sort_b);
-        int32_t *perm = (int32_t *)(base + sort_b + coords_b);
-        if (g->eval_dirty) {
-            if ((e = sgk_repack(g->d_alpha, g->d_blk, g->d_repack, g->L.S, st)) != cudaSuccess)
-                r = cuda_fail((cudaError_t)e, "repacking surpluses");
-            else
-                g->eval_dirty = 0;
+        if (need > have && parts) {
+            /* the segment sums do not fit: whole sums */
+            p.nshare = 1;
+            p.emit = SG_EMIT_SUM;
+            need = scratch_plan(m, g->L.d, sort, 0, &s);
         }
-        if (r == SG_OK) {
-            grid_plan(g, eval_ppt(g), &p);
-            /* the histogram is cleared inside the sort, so nothing left in
-             * the shared array by an earlier call is read */
-            if ((e = sgk_sort_points(coords, m, p.d, base, sorted, perm, st)) != cudaSuccess)
-                r = cuda_fail((cudaError_t)e, "sorting query points");
-            else if ((e = sgk_evaluate(&p, sorted, perm, out, m, st)) != cudaSuccess)
-                r = cuda_fail((cudaError_t)e, "evaluate");
-        }
+        if (need > have)
+            r = fail(SG_ERR_RANGE, "sg_evaluate_device_noalloc: %lld points in %d dims need more than the %lld-byte scratch",
+                     (long long)m, g->L.d, (long long)have);
+        else
+            r = evaluate_with(g, &p, &s, (char *)scratch, 0, coords, out, m, (cudaStream_t)stream);
     }
     leave(g, prev);
     return r;
@@ -926,50 +1017,15 @@ int sg_grid_prepare_eval(sg_grid *g, cudaStream_t st)
 {
     int e;
     if (!g->eval_dirty) return SG_OK;
-    if ((e = sgk_repack(g->d_alpha, g->d_blk, g->d_repack, g->L.S, st)) != cudaSuccess)
+    if ((e = sgk_repack(g->d_alpha, g->d_blk, g->d_repack, g->d_rsrc, g->L.nrows, g->L.n, st)) != cudaSuccess)
         return cuda_fail((cudaError_t)e, "repacking surpluses");
     g->eval_dirty = 0;
-    return SG_OK;
-}
-
-int sg_grid_set_parts(sg_grid *g, int nparts, cudaStream_t st)
-{
-    const sg_layout *L = &g->L;
-    uint32_t *tab;
-    int64_t words;
-    int r;
-    cudaError_t e;
-    if (nparts > SG_EVAL_MAX_PARTS) nparts = SG_EVAL_MAX_PARTS;
-    if (L->d < 4 || nparts <= 1 || g->dev < 0) {
-        g->nparts = 1;
-        return SG_OK;
-    }
-    words = 2 * (int64_t)(L->d - 2) * L->n;
-    tab = (uint32_t *)malloc((size_t)words * sizeof(uint32_t));
-    if (!tab) return fail(SG_ERR_NOMEM, "sg_grid_set_parts: out of host memory");
-    r = sg_layout_walk_tables(L, g->blk3, tab);
-    if (r == SG_OK) r = sg_layout_walk_split(L, nparts, g->split);
-    if (r == SG_OK && !g->d_walk) r = dev_alloc(g, (void **)&g->d_walk, words * 4, "walk tables");
-    if (r == SG_OK) {
-        /* pageable source: the copy has taken the bytes when the call returns */
-        e = cudaMemcpyAsync(g->d_walk, tab, (size_t)words * 4, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) r = cuda_fail(e, "uploading the walk tables");
-    }
-    free(tab);
-    if (r != SG_OK) return r;
-    g->nparts = nparts;
     return SG_OK;
 }
 
 void sg_grid_eval_args(const sg_grid *g, const float *coords, float *out, int64_t m, sg_eval_args *a)
 {
     sg_eval_plan p;
-    int k;
-    grid_plan(g, 2, &p);
+    grid_plan(g, &p);
     sgk_fill_eval_args(&p, coords, NULL, out, m, a);
-    if (g->nparts > 1) {
-        a->nparts = g->nparts;
-        for (k = 0; k <= g->nparts; k++) a->split[k] = g->split[k];
-        a->walk = g->d_walk;
-    }
 }

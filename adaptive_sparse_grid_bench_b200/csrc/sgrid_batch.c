@@ -68,7 +68,8 @@ SG_API int sg_batch_create(int num_grids, const int *dims, const int *levels, co
     b->voff = (int64_t *)calloc((size_t)num_grids + 1, sizeof(int64_t));
     b->doff = (int64_t *)calloc((size_t)num_grids + 1, sizeof(int64_t));
     b->boff = (int64_t *)calloc((size_t)num_grids + 1, sizeof(int64_t));
-    if (!b->L || !b->voff || !b->doff || !b->boff) {
+    b->seg_off = (int64_t *)calloc((size_t)num_grids, sizeof(int64_t));
+    if (!b->L || !b->voff || !b->doff || !b->boff || !b->seg_off) {
         sg_batch_destroy(b);
         return bfail(SG_ERR_NOMEM, "sg_batch_create: out of host memory");
     }
@@ -99,7 +100,6 @@ SG_API int sg_batch_create(int num_grids, const int *dims, const int *levels, co
         return bfail(SG_ERR_RANGE, "sg_batch_create: %lld values exceed 32-bit offsets", (long long)doff);
     }
     b->dev = -1;
-    b->ppt = 2;
     b->precision = SG_HIER_FP32;
     b->use_graph = 1;
     b->sort = 1;
@@ -120,6 +120,14 @@ static void free_dev(sg_batch *b)
     cudaFree(b->d_work);
     cudaFree(b->d_blk);
     cudaFree(b->d_repack);
+    cudaFree(b->d_rsrc);
+    cudaFree(b->d_seg);
+    cudaFree(b->d_part);
+    cudaFree(b->d_citems);
+    b->d_seg = NULL;
+    b->d_part = NULL;
+    b->d_citems = NULL;
+    b->part_floats = 0;
     cudaFree(b->d_smem_grids);
     cudaFree(b->d_smem_chains);
     cudaFree(b->d_smem_seg);
@@ -169,6 +177,7 @@ SG_API int sg_batch_destroy(sg_batch *b)
     free(b->voff);
     free(b->doff);
     free(b->boff);
+    free(b->seg_off);
     free(b->eval_pt_off);
     free(b->order);
     free(b);
@@ -264,6 +273,7 @@ static int materialize(sg_batch *b)
     uint32_t *segB[SG_MAX_DIMS];
     int64_t nchB[SG_MAX_DIMS], nsegB[SG_MAX_DIMS], capchB[SG_MAX_DIMS], capsegB[SG_MAX_DIMS];
     sg_repack *rp = NULL;
+    uint32_t *rs = NULL;
     int64_t nrp = 0;
     int64_t (*gfirst)[SG_MAX_DIMS] = NULL; /* first chain of each sweep group per sweep, ngroups+1 rows */
     int ngr = 0, capgr = 0, q;
@@ -459,25 +469,64 @@ static int materialize(sg_batch *b)
     }
 
     /* evaluation: repack table over all grids, per-grid block sizes */
-    for (g = 0; g < b->ng; g++) nrp += b->L[g].S;
-    rp = (sg_repack *)malloc((size_t)nrp * sizeof(sg_repack));
-    if (!rp) { r = bfail(SG_ERR_NOMEM, "out of host memory"); goto done; }
-    nrp = 0;
-    for (g = 0; g < b->ng; g++) {
-        sg_repack *one = NULL;
-        uint32_t blk3[SG_MAX_LEVELS], blk2[SG_MAX_LEVELS];
-        int64_t i;
-        if ((r = sg_layout_eval_tables(&b->L[g], &one, blk3, blk2)) != SG_OK) goto done;
-        for (i = 0; i < b->L[g].S; i++) {
-            rp[nrp + i] = one[i];
-            rp[nrp + i].src = (uint32_t)(one[i].src + b->doff[g]);
-            rp[nrp + i].dst = (uint32_t)(one[i].dst + b->boff[g]);
+    {
+        int64_t nsub = 0;
+        for (g = 0; g < b->ng; g++) {
+            nrp += b->L[g].nrows;
+            nsub += b->L[g].S;
+            if (b->L[g].n > b->max_n) b->max_n = b->L[g].n;
         }
-        nrp += b->L[g].S;
-        free(one);
+        rp = (sg_repack *)malloc((size_t)nrp * sizeof(sg_repack));
+        rs = (uint32_t *)malloc((size_t)nsub * sizeof(uint32_t));
+        if (!rp || !rs) { r = bfail(SG_ERR_NOMEM, "out of host memory"); goto done; }
+        nrp = nsub = 0;
+        for (g = 0; g < b->ng; g++) {
+            sg_repack *one = NULL;
+            uint32_t *off = NULL;
+            uint32_t blk3[SG_MAX_LEVELS], blk2[SG_MAX_LEVELS];
+            int64_t i;
+            if ((r = sg_layout_eval_tables(&b->L[g], &one, &off, blk3, blk2)) != SG_OK) goto done;
+            for (i = 0; i < b->L[g].nrows; i++) {
+                rp[nrp + i] = one[i];
+                rp[nrp + i].src = (uint32_t)(one[i].src + nsub);
+                rp[nrp + i].dst = (uint32_t)(one[i].dst + b->boff[g]);
+            }
+            for (i = 0; i < b->L[g].S; i++) rs[nsub + i] = (uint32_t)(off[i] + b->doff[g]);
+            nrp += b->L[g].nrows;
+            nsub += b->L[g].S;
+            free(one);
+            free(off);
+        }
+        b->nrepack = nrp;
+        /* segment tables of the grids that have one */
+        {
+            int64_t words = 0;
+            uint32_t *tab;
+            for (g = 0; g < b->ng; g++) {
+                b->seg_off[g] = sg_layout_seg_words(&b->L[g]) ? words : -1;
+                words += sg_layout_seg_words(&b->L[g]);
+            }
+            tab = (uint32_t *)malloc((size_t)(words > 0 ? words : 1) * 4);
+            if (!tab) { r = bfail(SG_ERR_NOMEM, "out of host memory"); goto done; }
+            for (g = 0; g < b->ng && r == SG_OK; g++) {
+                uint32_t blk3[SG_MAX_LEVELS];
+                int s;
+                if (b->seg_off[g] < 0) continue;
+                for (s = 0; s < b->L[g].n; s++) {
+                    sg_eval_shape sh;
+                    sg_layout_eval_shape(&b->L[g], s, &sh);
+                    blk3[s] = sh.coff[sh.cmax + 1];
+                }
+                r = sg_layout_seg_table(&b->L[g], blk3, tab + b->seg_off[g]);
+            }
+            if (r == SG_OK) r = upload(b, (void **)&b->d_seg, tab, words * 4, "batch segment tables");
+            else bfail(r, "building the segment tables");
+            free(tab);
+            if (r != SG_OK) goto done;
+        }
+        if ((r = upload(b, (void **)&b->d_repack, rp, nrp * (int64_t)sizeof(sg_repack), "batch repack table")) == SG_OK)
+            r = upload(b, (void **)&b->d_rsrc, rs, nsub * 4, "batch repack offsets");
     }
-    b->nrepack = nrp;
-    r = upload(b, (void **)&b->d_repack, rp, nrp * (int64_t)sizeof(sg_repack), "batch repack table");
 done:
     free(gfirst);
     free(order);
@@ -485,6 +534,7 @@ done:
     free(sch);
     free(sseg);
     free(rp);
+    free(rs);
     for (k = 0; k < SG_MAX_DIMS; k++) {
         free(chB[k]);
         free(segB[k]);
@@ -791,14 +841,6 @@ SG_API int sg_batch_hierarchize(sg_batch *b)
 /* Evaluation plan: per-grid kernel arguments and per-dimension CTA items for
  * the caller's point offsets and buffers (kept, so an identical call replays
  * the captured graph). */
-static int ppt_of(const sg_batch *b, int d) { return b->ppt_d[d] ? b->ppt_d[d] : b->ppt; }
-/* blocking preset index (0 .. SG_EVAL_BLOCKINGS-1) of dimension d */
-static int blk_of(const sg_batch *b, int d)
-{
-    const int v = b->blk_d[d] ? b->blk_d[d] : b->blocking;
-    return v > 0 ? v - 1 : 0;
-}
-
 static int cmp_dim_then_subspaces(const void *x, const void *y, void *ctx)
 {
     const sg_batch *b = (const sg_batch *)ctx;
@@ -881,12 +923,29 @@ out:
     return r;
 }
 
+#define SG_BATCH_SHARE_CTAS (8 * 296) /* launches with fewer CTAs share the sums of long chains */
+#define SG_BATCH_SHARE_CHAIN 512      /* subspaces per share to aim for (grids of one part)     */
+
+/* How many CTAs share the sums of a grid's points.  In a small batch the time
+ * is that of the longest chains (all S subspaces of a point in one thread); a
+ * large one hides them behind its other CTAs. */
+static int batch_shares(const sg_layout *L, int64_t ctas)
+{
+    const int nseg = sg_layout_segs(L), parts = sg_layout_parts(L);
+    int64_t n;
+    if (nseg <= 1 || ctas >= SG_BATCH_SHARE_CTAS) return 1;
+    if (parts > 1) return parts;
+    n = L->S / SG_BATCH_SHARE_CHAIN;
+    if (n > nseg) n = nseg;
+    return n < 1 ? 1 : (n > 8 ? 8 : (int)n);
+}
+
 static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, float *out)
 {
     int g, k, r, q;
-    int64_t coff = 0, ni = 0, cap_items = 0;
+    int64_t coff = 0, ni = 0, cap_items = 0, ctas = 0, parts = 0, nc = 0, cap_c = 0;
+    int32_t *citems;
     int same = b->h_eval_args && b->eval_coords == coords && b->eval_out == out && b->eval_sort == b->sort;
-    for (k = 0; same && k <= SG_MAX_DIMS; k++) same = b->eval_ppt_d[k] == ppt_of(b, k) && b->eval_blk_d[k] == blk_of(b, k);
     for (g = 0; same && g <= b->ng; g++) same = b->eval_pt_off[g] == pt_off[g];
     if (same) return SG_OK;
     if (b->eval_graph) {
@@ -900,12 +959,36 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
         if ((r = balloc(b, (void **)&b->d_eval_args, b->ng * (int64_t)sizeof(sg_eval_args), "batch eval args")) != SG_OK)
             return r;
     }
+    b->eval_pt_off[0] = -1; /* no plan until this one is complete */
     for (k = 0; k <= SG_MAX_DIMS; k++) b->items_first[k] = b->items_count[k] = 0;
     for (g = 0; g < b->ng; g++) {
         const int64_t m = pt_off[g + 1] - pt_off[g];
         if (m < 0) return bfail(SG_ERR_ARG, "sg_batch_evaluate: point offsets decrease at grid %d", g);
-        cap_items += (m + 255) / 256; /* enough for one point per thread */
+        ctas += (m + SG_EVAL_CTA_POINTS - 1) / SG_EVAL_CTA_POINTS;
     }
+    for (g = 0; g < b->ng; g++) {
+        const int64_t m = pt_off[g + 1] - pt_off[g];
+        const int ns = batch_shares(&b->L[g], ctas);
+        cap_items += (m + SG_EVAL_CTA_POINTS - 1) / SG_EVAL_CTA_POINTS * ns;
+        if (ns > 1) {
+            cap_c += (m + 255) / 256;
+            parts += m * (sg_layout_parts(&b->L[g]) > 1 ? sg_layout_parts(&b->L[g]) : sg_layout_segs(&b->L[g]));
+        }
+    }
+    if (parts > b->part_floats) {
+        cudaFree(b->d_part);
+        b->dev_bytes -= b->part_floats * 4;
+        b->d_part = NULL;
+        b->part_floats = 0;
+        r = balloc(b, (void **)&b->d_part, parts * 4, "batch segment sums");
+        if (r == SG_ERR_NOMEM) ctas = SG_BATCH_SHARE_CTAS; /* no room: whole sums need none */
+        else if (r != SG_OK) return r;
+        else b->part_floats = parts;
+    }
+    parts = 0;
+    for (k = 0; k <= SG_MAX_DIMS; k++) b->items_shared[k] = 0;
+    for (g = 0; g < b->ng; g++)
+        if (batch_shares(&b->L[g], ctas) > 1) b->items_shared[b->L[g].d] = 1;
     if (!b->order) {
         b->order = (int *)malloc(sizeof(int) * (size_t)b->ng);
         if (!b->order) return bfail(SG_ERR_NOMEM, "out of host memory");
@@ -935,8 +1018,13 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
                 p.blk3[s] = p.blk2[s] = 0;
             }
         }
-        p.ppt = ppt_of(b, L->d);
-        p.blocking = blk_of(b, L->d);
+        p.nseg = sg_layout_segs(L);
+        p.nparts = sg_layout_parts(L);
+        p.seg = b->seg_off[g] >= 0 ? b->d_seg + b->seg_off[g] : NULL;
+        p.nshare = batch_shares(L, ctas);
+        p.emit = p.nshare > 1 ? (p.nparts > 1 ? SG_EMIT_PARTS : SG_EMIT_SEGS) : SG_EMIT_SUM;
+        p.part_out = b->d_part + parts;
+        if (p.nshare > 1) parts += (pt_off[g + 1] - pt_off[g]) * (p.nparts > 1 ? p.nparts : p.nseg);
         sgk_fill_eval_args(&p, coords + coff, NULL, out + pt_off[g], pt_off[g + 1] - pt_off[g], &b->h_eval_args[g]);
         coff += (pt_off[g + 1] - pt_off[g]) * L->d;
     }
@@ -944,17 +1032,19 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
     /* items grouped by dimension, grids with the most subspaces first (their
      * CTAs are the longest) */
     for (k = 1; k <= SG_MAX_DIMS; k++) {
-        const int cta = 256 * ppt_of(b, k);
+        const int cta = SG_EVAL_CTA_POINTS;
         b->items_first[k] = (int)ni;
         for (q = 0; q < b->ng; q++) {
             int64_t st;
+            int sh;
             g = b->order[q];
             if (b->L[g].d != k) continue;
-            for (st = pt_off[g]; st < pt_off[g + 1]; st += cta) {
-                b->h_items[2 * ni] = g;
-                b->h_items[2 * ni + 1] = (int32_t)(st - pt_off[g]);
-                ni++;
-            }
+            for (st = pt_off[g]; st < pt_off[g + 1]; st += cta)
+                for (sh = 0; sh < b->h_eval_args[g].nshare; sh++) {
+                    b->h_items[2 * ni] = (int32_t)((uint32_t)g | ((uint32_t)sh << 29));
+                    b->h_items[2 * ni + 1] = (int32_t)(st - pt_off[g]);
+                    ni++;
+                }
         }
         b->items_count[k] = (int)ni - b->items_first[k];
     }
@@ -967,13 +1057,31 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
     BCU(cudaMemcpy(b->d_eval_args, b->h_eval_args, (size_t)b->ng * sizeof(sg_eval_args), cudaMemcpyHostToDevice),
         "upload eval args");
     if (ni > 0) BCU(cudaMemcpy(b->d_items, b->h_items, (size_t)ni * 2 * 4, cudaMemcpyHostToDevice), "upload items");
+    /* combine CTAs of the grids with shared sums */
+    cudaFree(b->d_citems);
+    b->d_citems = NULL;
+    b->dev_bytes -= (int64_t)b->ncitems * 8;
+    b->ncitems = 0;
+    if (cap_c > 0) {
+        citems = (int32_t *)malloc((size_t)cap_c * 8);
+        if (!citems) return bfail(SG_ERR_NOMEM, "out of host memory");
+        for (g = 0; g < b->ng; g++) {
+            int64_t p;
+            if (b->h_eval_args[g].nshare <= 1) continue;
+            for (p = 0; p < pt_off[g + 1] - pt_off[g]; p += 256) {
+                citems[2 * nc] = g;
+                citems[2 * nc + 1] = (int32_t)p;
+                nc++;
+            }
+        }
+        r = upload(b, (void **)&b->d_citems, citems, nc * 8, "batch combine items");
+        free(citems);
+        if (r != SG_OK) return r;
+        b->ncitems = (int)nc;
+    }
     for (g = 0; g <= b->ng; g++) b->eval_pt_off[g] = pt_off[g];
     b->eval_coords = coords;
     b->eval_out = out;
-    for (k = 0; k <= SG_MAX_DIMS; k++) {
-        b->eval_ppt_d[k] = ppt_of(b, k);
-        b->eval_blk_d[k] = blk_of(b, k);
-    }
     b->eval_sort = b->sort;
     return SG_OK;
 }
@@ -999,18 +1107,20 @@ static int eval_launches(sg_batch *b, cudaStream_t st)
                                               b->sort_nbins, b->d_sscratch, b->d_sorted, b->d_perm, st)) !=
                        cudaSuccess)
         return bcuda((cudaError_t)e, "batch spatial ordering");
-    if ((e = sgk_repack(b->d_alpha, b->d_blk, b->d_repack, b->nrepack, st)) != cudaSuccess)
+    if ((e = sgk_repack(b->d_alpha, b->d_blk, b->d_repack, b->d_rsrc, b->nrepack, b->max_n, st)) != cudaSuccess)
         return bcuda((cudaError_t)e, "batch repack");
     BCU(cudaEventRecord(b->ev_fork, st), "cudaEventRecord");
     for (k = 1; k <= SG_MAX_DIMS; k++) {
         if (!b->items_count[k]) continue;
         BCU(cudaStreamWaitEvent(b->dst[k], b->ev_fork, 0), "cudaStreamWaitEvent");
         e = sgk_evaluate_batch(k, b->d_eval_args, b->d_items + 2 * (int64_t)b->items_first[k], b->items_count[k],
-                               ppt_of(b, k), blk_of(b, k), b->dst[k]);
+                               b->items_shared[k], b->dst[k]);
         if (e != cudaSuccess) return bcuda((cudaError_t)e, "batch evaluate");
         BCU(cudaEventRecord(b->ev_d[k], b->dst[k]), "cudaEventRecord");
         BCU(cudaStreamWaitEvent(st, b->ev_d[k], 0), "cudaStreamWaitEvent");
     }
+    if (b->ncitems && (e = sgk_combine_parts(b->d_eval_args, b->d_citems, b->ncitems, st)) != cudaSuccess)
+        return bcuda((cudaError_t)e, "batch segment sums");
     return SG_OK;
 }
 
@@ -1037,7 +1147,7 @@ SG_API int sg_batch_autotune(sg_batch *b, const int64_t *point_offsets, const fl
     cudaStream_t st = (cudaStream_t)stream;
     cudaEvent_t e0 = NULL, e1 = NULL;
     double t[2 * SG_EVAL_BLOCKINGS][SG_MAX_DIMS + 1];
-    int prev, r, pi, k, q, rep, cfg;
+    int prev, r, k, q, rep, cfg;
     float el;
     if (!b || !point_offsets || point_offsets[0] != 0) return bfail(SG_ERR_ARG, "sg_batch_autotune: bad argument");
     if (!b->has_values || b->dev < 0) return bfail(SG_ERR_STATE, "sg_batch_autotune: no values have been set");
@@ -1050,21 +1160,16 @@ SG_API int sg_batch_autotune(sg_batch *b, const int64_t *point_offsets, const fl
         goto done;
     }
     if ((r = make_fork_streams(b)) != SG_OK) goto done;
-    /* every dimension's launch alone on st, at 1 and at 2 points per thread
-     * (pi) under each blocking preset (cfg / 2) */
+    /* every dimension's launch alone on st, once per setting of points per
+     * thread and blocking (the kernels have one form) */
     for (cfg = 0; cfg < 2 * SG_EVAL_BLOCKINGS && r == SG_OK; cfg++) {
-        pi = cfg % 2;
-        for (k = 0; k <= SG_MAX_DIMS; k++) {
-            b->ppt_d[k] = pi + 1;
-            b->blk_d[k] = cfg / 2 + 1;
-        }
         if ((r = plan_eval(b, point_offsets, coords, out)) != SG_OK) break;
         if (b->sort && sgk_batch_sort_points(coords, b->d_sgrids, b->d_sitems, b->nsitems, b->sort_npts, b->sort_nbins,
                                              b->d_sscratch, b->d_sorted, b->d_perm, st) != cudaSuccess) {
             r = bfail(SG_ERR_CUDA, "sg_batch_autotune: spatial ordering");
             break;
         }
-        if (sgk_repack(b->d_alpha, b->d_blk, b->d_repack, b->nrepack, st) != cudaSuccess) {
+        if (sgk_repack(b->d_alpha, b->d_blk, b->d_repack, b->d_rsrc, b->nrepack, b->max_n, st) != cudaSuccess) {
             r = bfail(SG_ERR_CUDA, "sg_batch_autotune: repack");
             break;
         }
@@ -1073,7 +1178,7 @@ SG_API int sg_batch_autotune(sg_batch *b, const int64_t *point_offsets, const fl
             for (rep = 0; rep < 3; rep++) { /* first run warms */
                 if (cudaEventRecord(e0, st) != cudaSuccess ||
                     sgk_evaluate_batch(k, b->d_eval_args, b->d_items + 2 * (int64_t)b->items_first[k],
-                                       b->items_count[k], pi + 1, cfg / 2, st) != cudaSuccess ||
+                                       b->items_count[k], b->items_shared[k], st) != cudaSuccess ||
                     cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                     cudaEventElapsedTime(&el, e0, e1) != cudaSuccess) {
                     r = bfail(SG_ERR_CUDA, "sg_batch_autotune: timing d=%d", k);
@@ -1082,13 +1187,6 @@ SG_API int sg_batch_autotune(sg_batch *b, const int64_t *point_offsets, const fl
                 if (rep > 0 && (t[cfg][k] < 0.0 || el < t[cfg][k])) t[cfg][k] = el;
             }
         }
-    }
-    for (k = 0; k <= SG_MAX_DIMS; k++) {
-        int best = -1;
-        for (cfg = 0; r == SG_OK && cfg < 2 * SG_EVAL_BLOCKINGS; cfg++)
-            if (t[cfg][k] >= 0.0 && (best < 0 || t[cfg][k] < t[best][k])) best = cfg;
-        b->ppt_d[k] = best >= 0 ? best % 2 + 1 : 0;
-        b->blk_d[k] = best >= 0 ? best / 2 + 1 : 0;
     }
     b->eval_dirty = 1;
     /* sweeps: per chain size class, the staged chain kernel or one warp per
@@ -1166,15 +1264,11 @@ SG_API int sg_batch_set_option(sg_batch *b, int option, int64_t value)
         return SG_OK;
     case SG_OPT_EVAL_PPT:
         if (value < 0 || value > 2) return bfail(SG_ERR_ARG, "SG_OPT_EVAL_PPT is 0, 1 or 2");
-        b->ppt = value == 0 ? 2 : (int)value;
-        memset(b->ppt_d, 0, sizeof(b->ppt_d)); /* an explicit setting replaces tuned ones */
-        return SG_OK;
+        return SG_OK; /* one kernel form */
     case SG_OPT_EVAL_BLOCKING:
         if (value < 0 || value > SG_EVAL_BLOCKINGS)
             return bfail(SG_ERR_ARG, "SG_OPT_EVAL_BLOCKING is 0 .. %d", SG_EVAL_BLOCKINGS);
-        b->blocking = (int)value;
-        memset(b->blk_d, 0, sizeof(b->blk_d));
-        return SG_OK;
+        return SG_OK; /* one kernel form */
     case SG_OPT_USE_GRAPH:
         if (value != 0 && value != 1) return bfail(SG_ERR_ARG, "SG_OPT_USE_GRAPH is 0 or 1");
         b->use_graph = (int)value;

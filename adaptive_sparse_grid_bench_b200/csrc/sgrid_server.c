@@ -53,9 +53,6 @@
 #define SRV_HEAVY_PAIRS ((int64_t)1 << 27) /* default SG_SRV_OPT_HEAVY_PAIRS */
 #define SRV_MAX_REQS 8192 /* requests per batch */
 #define SRV_CTA_THREADS 256
-#define SRV_SPLIT_SUBSPACES 4096  /* grids (d >= 4) with this many subspaces get split sums */
-#define SRV_PART_SUBSPACES 2048   /* about this many subspaces per part (at most 8 parts) */
-#define SRV_LONG_CHAIN 2048       /* light launches with a part this long use 1 point per thread */
 #define SRV_WHOLE_POINTS 8192     /* heavy requests with this many points are not split: their
                                      own points give the launch enough CTAs */
 #define SRV_RING_BATCHES 4        /* the staging ring holds this many full batches */
@@ -375,7 +372,7 @@ static int take_batch(sg_server *s, srv_slot *sl)
         sl->out_off[sl->nreq] = pts;
         sl->coord_off[sl->nreq] = coff;
         sl->part_off[sl->nreq] = poff;
-        if (r->g->nparts > 1 && !whole_sums(r)) poff += r->m * r->g->nparts;
+        if (sg_layout_parts(&r->g->L) > 1 && !whole_sums(r)) poff += r->m * sg_layout_parts(&r->g->L);
         coff += r->m * r->d;
         pts += r->m;
         sl->nreq++;
@@ -401,7 +398,7 @@ static int launch_batch(sg_server *s, srv_slot *sl)
 {
     int64_t coff = 0, pts = 0, ni = 0, nc = 0;
     int i, d, e, no = 0;
-    int first[SG_MAX_DIMS + 1], count[SG_MAX_DIMS + 1], ppt[SG_MAX_DIMS + 1];
+    int first[SG_MAX_DIMS + 1], count[SG_MAX_DIMS + 1], shared[SG_MAX_DIMS + 1];
     const int zc = sl->zero_copy; /* fixed for the batch when it was taken */
     const int sort = sl->sort;    /* heavy lane: spatial ordering of each request's points */
     for (i = 0; i < sl->nreq; i++) {
@@ -422,11 +419,9 @@ static int launch_batch(sg_server *s, srv_slot *sl)
         }
         sg_grid_eval_args(r->g, dc, (zc ? sl->m_out : sl->d_out) + sl->out_off[i], r->m, &sl->h_args[i]);
         if (sort) sl->h_args[i].perm = sl->d_perm + sl->out_off[i];
-        if (whole_sums(r)) {
-            sl->h_args[i].nparts = 1;
-            sl->h_args[i].part_out = NULL;
-        }
-        if (sl->h_args[i].nparts > 1) {
+        if (sl->h_args[i].nparts > 1 && !whole_sums(r)) {
+            sl->h_args[i].nshare = sl->h_args[i].nparts;
+            sl->h_args[i].emit = SG_EMIT_PARTS;
             sl->h_args[i].part_out = sl->d_part + sl->part_off[i];
             for (p = 0; p < r->m; p += SRV_CTA_THREADS) {
                 sl->h_citems[2 * nc] = i;
@@ -439,22 +434,19 @@ static int launch_batch(sg_server *s, srv_slot *sl)
     }
     for (d = 1; d <= SG_MAX_DIMS; d++) {
         const int lo = no;
-        int64_t chain = 0, cta;
         first[d] = (int)ni;
+        shared[d] = 0;
         for (i = 0; i < sl->nreq; i++)
             if (sl->reqs[i]->d == d) {
-                const int64_t c = sl->reqs[i]->S / sl->h_args[i].nparts;
                 sl->order[no++] = i;
-                if (c > chain) chain = c;
+                shared[d] |= sl->h_args[i].nshare > 1;
             }
         sort_by_subspaces(sl, lo, no);
-        ppt[d] = (sl->lane == 0 && chain >= SRV_LONG_CHAIN) ? 1 : 2;
-        cta = (int64_t)SRV_CTA_THREADS * ppt[d];
         for (i = lo; i < no; i++) {
-            const int q = sl->order[i], np = sl->h_args[q].nparts;
+            const int q = sl->order[i], np = sl->h_args[q].nshare;
             int64_t p;
             int k;
-            for (p = 0; p < sl->reqs[q]->m; p += cta)
+            for (p = 0; p < sl->reqs[q]->m; p += SG_EVAL_CTA_POINTS)
                 for (k = 0; k < np; k++) {
                     sl->h_items[2 * ni] = q | (k << 29);
                     sl->h_items[2 * ni + 1] = (int32_t)p;
@@ -482,7 +474,7 @@ static int launch_batch(sg_server *s, srv_slot *sl)
     for (d = 1; d <= SG_MAX_DIMS; d++) {
         if (!count[d]) continue;
         if (cudaStreamWaitEvent(sl->dst[d], sl->ev_in, 0) != cudaSuccess) return SG_ERR_CUDA;
-        e = sgk_evaluate_batch(d, sl->d_args, sl->d_items + 2 * (int64_t)first[d], count[d], ppt[d], 0, sl->dst[d]);
+        e = sgk_evaluate_batch(d, sl->d_args, sl->d_items + 2 * (int64_t)first[d], count[d], shared[d], sl->dst[d]);
         if (e != cudaSuccess || cudaEventRecord(sl->ev_d[d], sl->dst[d]) != cudaSuccess ||
             cudaStreamWaitEvent(sl->st, sl->ev_d[d], 0) != cudaSuccess)
             return SG_ERR_CUDA;
@@ -776,7 +768,7 @@ SG_API int sg_server_destroy(sg_server *s)
  * tables), from its host layout */
 static int64_t grid_bytes_estimate(const sg_layout *L)
 {
-    return L->Npad * 4 + L->Nblk * 4 + L->S * (int64_t)(sizeof(sg_repack) + 12 * L->d) + (1 << 16);
+    return L->Npad * 4 + L->Nblk * 4 + L->nrows * (int64_t)sizeof(sg_repack) + L->S * (int64_t)(4 + 12 * L->d) + (1 << 16);
 }
 
 /* Evicts the least recently used grid that no request needs (lock held);
@@ -806,10 +798,6 @@ static int build_grid(sg_server *s, int d, int n, const int *limits, int fn, con
     if (r == SG_OK) r = sg_sample_function(g, fn, params, num_params, s->admit_st);
     if (r == SG_OK) r = sg_hierarchize_async(g, s->admit_st);
     if (r == SG_OK) r = sg_grid_prepare_eval(g, s->admit_st);
-    if (r == SG_OK && d >= 4 && g->L.S >= SRV_SPLIT_SUBSPACES) {
-        const int64_t np = g->L.S / SRV_PART_SUBSPACES;
-        r = sg_grid_set_parts(g, np > SG_EVAL_MAX_PARTS ? SG_EVAL_MAX_PARTS : (int)np, s->admit_st);
-    }
     if (r == SG_OK) r = sg_sync(g, s->admit_st);
     if (r != SG_OK) {
         if (g) {

@@ -59,8 +59,11 @@ extern "C" {
 /* Options (sg_set_option / sg_get_option). */
 #define SG_OPT_HIER_PRECISION 1 /* SG_HIER_FP32 (default) or SG_HIER_FP64           */
 #define SG_OPT_EVAL_SORT 2      /* 1 (default): spatially order points on the GPU   */
-                                /* before evaluating; 0: evaluate in caller order    */
-#define SG_OPT_EVAL_PPT 3       /* points per thread in evaluate: 0 = auto, 1, 2     */
+                                /* before evaluating where that pays (enough points, */
+                                /* a grid beyond L1); 0: evaluate in caller order    */
+#define SG_OPT_EVAL_PPT 3       /* 0, 1 or 2, without effect: every thread takes two */
+                                /* points, and few points share their sums among     */
+                                /* warps                                             */
 #define SG_OPT_HIER_KERNEL 5    /* 0 = auto, 1 = shared-memory chains, 2 = gather,   */
                                 /* 3 = one warp per chain (batches only)            */
 #define SG_OPT_PROFILE 6        /* 1: record CUDA events around each phase            */
@@ -75,14 +78,8 @@ extern "C" {
                                 /* k * 2^20 clock cycles (about k/2 ms); the next     */
                                 /* sg_sync returns SG_ERR_TIMEOUT and the values are  */
                                 /* invalid.  0 (default): off.                       */
-#define SG_OPT_EVAL_BLOCKING 10 /* evaluate: how much of the subspace walk runs as   */
-                                /* fully unrolled blocks of compile-time shape:      */
-                                /* 1 = wide (3-D blocks of level budget <= 6, leaf  */
-                                /* subtrees of budget <= 5 at one point per thread  */
-                                /* or <= 4 at two), 2 = medium (5, 3); 0 = auto    */
-                                /* (wide, or the tuned choice).  Grids of d < 3 or  */
-                                /* d > 12 have one form.  Results are bit-identical */
-                                /* under every setting.                             */
+#define SG_OPT_EVAL_BLOCKING 10 /* 0, 1 or 2, without effect: the kernels have one   */
+                                /* form                                              */
 
 /* Phases reported by sg_timings (milliseconds of the most recent call). */
 #define SG_PHASE_HIERARCHIZE 0  /* all sweeps of the last hierarchization    */
@@ -160,9 +157,9 @@ int sg_sync(sg_grid *grid, void *stream);
 
 /* Autotuner (no reference counterpart; the reference tunes its CUDA block
  * size by hand, run.sh).  Times, on the caller's device buffers and stream,
- * the evaluation under every setting of points per thread {1, 2} x spatial
- * ordering {off, on}, then, at the faster of those, under every subspace
- * blocking (SG_OPT_EVAL_BLOCKING 1..2), and the hierarchization with the
+ * the evaluation under every setting of SG_OPT_EVAL_PPT {1, 2} x spatial
+ * ordering {off, on}, then, at the faster of those, under every value of
+ * SG_OPT_EVAL_BLOCKING (1..2), and the hierarchization with the
  * shared-memory chain sweeps (where they fit) and the gather sweeps; keeps
  * the fastest in the handle's options (SG_OPT_EVAL_PPT, SG_OPT_EVAL_SORT,
  * SG_OPT_EVAL_BLOCKING, SG_OPT_HIER_KERNEL).  No setting changes any result.
@@ -258,14 +255,12 @@ int sg_batch_sync(sg_batch *batch, void *stream);
  * SG_ERR_STATE after it) */
 int sg_batch_set_option(sg_batch *batch, int option, int64_t value);
 /* Autotuner for batches (no reference counterpart): times each
- * dimension's evaluation launch over the caller's points at 1 and at 2
- * points per thread under each subspace blocking (SG_OPT_EVAL_BLOCKING
- * 1..2) and keeps the fastest pair per dimension, and times the
- * hierarchization with each chain size class on the staged chain kernel and
+ * dimension's evaluation launch over the caller's points once per setting of
+ * SG_OPT_EVAL_PPT and SG_OPT_EVAL_BLOCKING (the kernels have one form: for
+ * information), and times the hierarchization with each chain size class on the staged chain kernel and
  * on one warp per chain and keeps the faster per class (the values are
- * saved and restored).  Results do not change.  An SG_OPT_EVAL_PPT,
- * SG_OPT_EVAL_BLOCKING or SG_OPT_HIER_KERNEL setting replaces the tuned
- * choice.  ms (optional, SG_BATCH_TUNE_TIMINGS entries):
+ * saved and restored).  Results do not change.  An SG_OPT_HIER_KERNEL
+ * setting replaces the tuned choice.  ms (optional, SG_BATCH_TUNE_TIMINGS entries):
  * [(blocking-1)*2 + ppt-1][d] launch ms, -1 where no grid has d. */
 #define SG_BATCH_TUNE_TIMINGS (4 * (SG_MAX_DIMS + 1))
 int sg_batch_autotune(sg_batch *batch, const int64_t *point_offsets, const float *coord_mat, float *out,
