@@ -393,6 +393,42 @@ __global__ void k_copy_segments(const float *__restrict__ src, float *__restrict
     }
 }
 
+/* Moves a grid's first level groups between the caller's compact array and
+ * the group-aligned layout in one launch.  Groups start on multiples of 32 in the
+ * layout, so a warp's 32 consecutive places lie in one group; the largest group
+ * is the last, so it is looked for from the end. */
+struct GroupTables {
+    int n;
+    int64_t compact[SG_MAX_LEVELS + 1], dev[SG_MAX_LEVELS + 1];
+};
+__global__ void __launch_bounds__(256) k_copy_groups(const float *__restrict__ src, float *__restrict__ dst,
+                                                     const GroupTables T, int64_t npad, int to_compact)
+{
+    constexpr int kSteps = 4; /* 8: 69 us instead of 65 at d = 10, n = 10 */
+    const int64_t step = (int64_t)gridDim.x * 256;
+    for (int64_t i0 = blockIdx.x * (int64_t)256 + threadIdx.x; i0 < npad; i0 += kSteps * step) {
+        float v[kSteps];
+        int64_t to[kSteps];
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k) {
+            const int64_t i = i0 + k * step;
+            to[k] = -1;
+            if (i < npad) {
+                int s = T.n - 1;
+                while (i < T.dev[s]) --s;
+                const int64_t c = T.compact[s] + (i - T.dev[s]);
+                if (c < T.compact[s + 1]) { /* not padding */
+                    v[k] = src[to_compact ? i : c];
+                    to[k] = to_compact ? c : i;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k)
+            if (to[k] >= 0) dst[to[k]] = v[k];
+    }
+}
+
 int g_num_sms = 0;
 long long g_launches = 0;
 
@@ -619,6 +655,22 @@ int sgk_copy_segments(const float *src, float *dst, const sg_copy_seg *segs, int
     if (nseg <= 0) return cudaSuccess;
     int64_t g = nseg < 148 * 32 ? nseg : 148 * 32;
     k_copy_segments<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(src, dst, segs, nseg, to_compact);
+    sgk_count(1);
+    return cudaGetLastError();
+}
+
+int sgk_copy_groups(const sg_layout *L, int groups, const float *src, float *dst, int to_compact, void *stream)
+{
+    GroupTables T;
+    if (groups <= 0) return cudaSuccess;
+    T.n = groups;
+    for (int s = 0; s <= SG_MAX_LEVELS; ++s) {
+        T.compact[s] = L->lidx[s <= groups ? s : groups];
+        T.dev[s] = L->plidx[s <= groups ? s : groups];
+    }
+    int64_t g = (L->plidx[groups] + 1023) / 1024;
+    if (g > 148 * 8) g = 148 * 8;
+    k_copy_groups<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(src, dst, T, L->plidx[groups], to_compact);
     sgk_count(1);
     return cudaGetLastError();
 }

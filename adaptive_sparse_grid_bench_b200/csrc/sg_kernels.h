@@ -58,6 +58,8 @@ typedef struct sg_copy_seg {
 int sgk_copy_segments(const float *src, float *dst, const sg_copy_seg *segs, int64_t nseg, int to_compact,
                       void *stream);
 int sgk_narrow(const double *src, float *dst, int64_t n, void *stream);
+/* The same for the first `groups` level groups of one grid, from its layout alone. */
+int sgk_copy_groups(const sg_layout *L, int groups, const float *src, float *dst, int to_compact, void *stream);
 
 /* Evaluation. */
 typedef struct sg_eval_plan {
