@@ -19,6 +19,18 @@
 typedef int (*sg_dev_alloc_fn)(void *ctx, void **ptr, int64_t bytes);
 typedef void (*sg_dev_free_fn)(void *ctx, void *ptr);
 
+/* A pass of the hierarchization: the sweeps of p.g dims from k0 on, or (p.g =
+ * 0) the single-dim sweep of k0. */
+typedef struct sg_pass_state {
+    sg_unit_pass p;
+    int k0;
+    sg_unit *units;
+    uint32_t *offs;
+    sg_unit_combo *combos;
+    sg_unit_node *nodes;
+    uint16_t *combo_of;
+} sg_pass_state;
+
 struct sg_grid {
     sg_layout L;
     int dev;        /* device of the device state, -1 before it exists */
@@ -35,6 +47,8 @@ struct sg_grid {
     sg_chain *d_chains[SG_MAX_DIMS];
     uint32_t *d_seg[SG_MAX_DIMS];
     sg_sweep_tables sweep[SG_MAX_DIMS];
+    sg_pass_state pass[2][SG_MAX_DIMS]; /* FP32, FP64: the sweeps in order, built when first called for */
+    int npass[2];
     int *d_err;       /* device-side wait timeout flag             */
     void *d_scratch;  /* evaluate: sort scratch + sorted coords + permutation */
     int64_t scratch_bytes;

@@ -46,6 +46,16 @@ int sgk_sweep_gather_f64(double *a, const sg_sweep_tables *t, void *stream);
 int sgk_sweep_small_f32(float *a, const sg_sweep_tables *t, void *stream);
 int sgk_sweep_small_f64(double *a, const sg_sweep_tables *t, void *stream);
 int64_t sgk_small_smem_bytes(int64_t cap_elems, int elem_bytes);
+/* The sweeps of g consecutive dims in one pass (hier_fused.cu). */
+typedef struct sg_unit_pass {
+    const sg_unit *units;  /* device */
+    const uint32_t *offs;  /* device */
+    int64_t nunits, max_elems;
+    int g;
+    sg_unit_tables tables;
+} sg_unit_pass;
+int sgk_sweep_fused_f32(float *a, const sg_unit_pass *p, void *stream);
+int sgk_sweep_fused_f64(double *a, const sg_unit_pass *p, void *stream);
 int sgk_widen(const float *src, double *dst, int64_t n, void *stream);
 
 /* A run of values at `compact` in a caller's compact array and at `dev` in

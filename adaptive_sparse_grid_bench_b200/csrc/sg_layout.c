@@ -216,6 +216,231 @@ int sg_layout_chains(const sg_layout *L, int k, sg_chain **chains, int64_t *ncha
     return SG_OK;
 }
 
+/* ---- passes of several sweeps -------------------------------------------- */
+
+/* nodes of the grid of dims k0..k0+g-1 with budget R */
+static int64_t pass_nodes(const sg_layout *L, int k0, int g, int R)
+{
+    int64_t c[SG_MAX_LEVELS], t = 0;
+    int i, s, l;
+    for (s = 0; s <= R; s++) c[s] = s == 0;
+    for (i = k0; i < k0 + g; i++)
+        for (s = R; s >= 0; s--) {
+            int64_t v = 0;
+            for (l = 0; l <= s && l <= L->lim[i]; l++) v += c[s - l];
+            c[s] = v;
+        }
+    for (s = 0; s <= R; s++) t += c[s] << s;
+    return t;
+}
+
+int sg_layout_pass_dims(const sg_layout *L, int k0, int elem_bytes)
+{
+    const int most = L->d - k0 < 3 ? L->d - k0 : 3;
+    int g, R;
+    /* a single dim gains nothing over the single-dim sweep, except as the
+     * rest of a grid that is otherwise done in passes */
+    for (g = most; g >= (k0 > 0 ? 1 : 2); g--) {
+        /* the largest unit's nodes: one CTA works through them, so three dims
+         * only where that is short (n <= 6), two up to n = 10, and only where it
+         * is a small part of the grid (d >= 5 or so) */
+        const int64_t nodes = pass_nodes(L, k0, g, L->n - 1);
+        int64_t elems = 0;
+        if (nodes > (g == 3 ? SG_PASS3_NODES : SG_PASS_NODES) || 16 * nodes > L->N) continue;
+        for (R = 1; R < L->n; R++) {
+            const int64_t e = pass_nodes(L, k0, g, R) * sgk_unit_stride(L->n - 1 - R);
+            if (e > elems) elems = e;
+        }
+        if (elems * elem_bytes <= (g == 1 ? SG_PASS1_BYTES : SG_UNIT_MAX_BYTES)) return g;
+    }
+    return 0;
+}
+
+void sg_layout_pass_free(sg_pass_host *p)
+{
+    free(p->units);
+    free(p->offs);
+    free(p->combos);
+    free(p->nodes);
+    free(p->combo_of);
+    memset(p, 0, sizeof(*p));
+}
+
+typedef struct {
+    const sg_layout *L;
+    sg_pass_host *p;
+    int k0, g;
+    int64_t cap_u, cap_o;
+    int err;
+} unit_ctx;
+
+static void unit_visit(void *vctx, int *lv, int sigma)
+{
+    unit_ctx *c = (unit_ctx *)vctx;
+    const sg_layout *L = c->L;
+    sg_pass_host *p = c->p;
+    const int R = L->n - 1 - sigma;
+    int i, m, lo = 0, nc;
+    int64_t e;
+    if (c->err || R < 1) return;
+    nc = p->tables.ncombo[R];
+    if (nc < 2) return; /* limits leave nothing to sweep */
+    if (p->nunits == c->cap_u) {
+        void *q;
+        c->cap_u = c->cap_u ? 2 * c->cap_u : 1024;
+        q = realloc(p->units, (size_t)c->cap_u * sizeof(sg_unit));
+        if (!q) { c->err = SG_ERR_NOMEM; return; }
+        p->units = (sg_unit *)q;
+    }
+    while (p->noffs + nc > c->cap_o) {
+        void *q;
+        c->cap_o = c->cap_o ? 2 * c->cap_o : 4096;
+        q = realloc(p->offs, (size_t)c->cap_o * sizeof(uint32_t));
+        if (!q) { c->err = SG_ERR_NOMEM; return; }
+        p->offs = (uint32_t *)q;
+    }
+    for (m = c->k0 + c->g; m < L->d; m++) lo += lv[m];
+    p->units[p->nunits].off = (uint32_t)p->noffs;
+    p->units[p->nunits].R = (uint8_t)R;
+    p->units[p->nunits].sigma = (uint8_t)sigma;
+    p->units[p->nunits].lo = (uint8_t)lo;
+    p->units[p->nunits].pad = 0;
+    p->nunits++;
+    for (i = 0; i < nc; i++) {
+        for (m = 0; m < c->g; m++) lv[c->k0 + m] = p->combos[i].lv[m];
+        p->offs[p->noffs++] = (uint32_t)sg_layout_subspace_offset(L, lv);
+    }
+    for (m = 0; m < c->g; m++) lv[c->k0 + m] = 0;
+    i = nc - 1;
+    e = ((int64_t)p->combos[i].node + ((int64_t)1 << p->combos[i].sum)) * sgk_unit_stride(sigma);
+    if (e > p->max_elems) p->max_elems = e;
+}
+
+/* largest budgets first: their CTAs run longest */
+static int unit_cmp(const void *a, const void *b)
+{
+    const sg_unit *x = (const sg_unit *)a, *y = (const sg_unit *)b;
+    if (x->R != y->R) return x->R > y->R ? -1 : 1;
+    return x->off < y->off ? -1 : (x->off > y->off);
+}
+
+/* the 1-D parent of index i at level j on one side: -1 at the boundary */
+static int parent_of(int i, int j, int side, int *level)
+{
+    int m = i + side, tz = 0;
+    if (m == 0 || m == (1 << j)) return -1;
+    while (!((m >> tz) & 1)) tz++;
+    *level = j - 1 - tz;
+    return m >> (tz + 1);
+}
+
+int sg_layout_pass(const sg_layout *L, int k0, int g, sg_pass_host *p)
+{
+    int id[SG_MAX_LEVELS][SG_MAX_LEVELS][SG_MAX_LEVELS];
+    int dims[SG_MAX_DIMS], lv[SG_MAX_DIMS], lim[3], m = 0, i, q, s, a, b, c;
+    uint32_t fill[3][SG_MAX_LEVELS];
+    sg_unit_tables *t = &p->tables;
+    unit_ctx ctx;
+    int64_t node = 0, total = 0;
+    memset(p, 0, sizeof(*p));
+    for (q = 0; q < 3; q++) {
+        lim[q] = q < g ? L->lim[k0 + q] : 0;
+        t->lmax[q] = lim[q];
+    }
+    /* combos by level sum */
+    p->combos = (sg_unit_combo *)malloc(sizeof(sg_unit_combo) * SG_MAX_LEVELS * SG_MAX_LEVELS * SG_MAX_LEVELS);
+    if (!p->combos) return SG_ERR_NOMEM;
+    for (s = 0; s < L->n; s++) {
+        for (a = 0; a <= s && a <= lim[0]; a++)
+            for (b = 0; a + b <= s && b <= lim[1]; b++) {
+                c = s - a - b;
+                if (c > lim[2]) continue;
+                id[a][b][c] = (int)p->ncombos;
+                p->combos[p->ncombos].lv[0] = (uint8_t)a;
+                p->combos[p->ncombos].lv[1] = (uint8_t)b;
+                p->combos[p->ncombos].lv[2] = (uint8_t)c;
+                p->combos[p->ncombos].sum = (uint8_t)s;
+                p->combos[p->ncombos].node = (uint32_t)node;
+                p->ncombos++;
+                node += (int64_t)1 << s;
+            }
+        t->ncombo[s] = (int)p->ncombos;
+        t->nnode[s] = (int)node;
+    }
+    if (node > SG_UNIT_NONE) return SG_ERR_RANGE;
+    p->nall = node;
+    p->combo_of = (uint16_t *)malloc(sizeof(uint16_t) * (size_t)node);
+    if (!p->combo_of) return SG_ERR_NOMEM;
+    for (m = 0; m < p->ncombos; m++)
+        for (i = 0; i < 1 << p->combos[m].sum; i++) p->combo_of[p->combos[m].node + (uint32_t)i] = (uint16_t)m;
+    /* lists of the points of level j in dim q, in node order (so by level sum) */
+    for (q = 0; q < g; q++)
+        for (i = 1; i <= lim[q]; i++) {
+            uint32_t run = 0;
+            t->first[q][i] = fill[q][i] = (uint32_t)total;
+            for (s = 0; s < L->n; s++) {
+                for (m = s ? t->ncombo[s - 1] : 0; m < t->ncombo[s]; m++)
+                    if (p->combos[m].lv[q] == i) run += 1u << s;
+                t->count[q][i][s] = (uint16_t)run;
+            }
+            total += run;
+        }
+    p->nnodes = total;
+    p->nodes = (sg_unit_node *)malloc(sizeof(sg_unit_node) * (size_t)(total > 0 ? total : 1));
+    if (!p->nodes) return SG_ERR_NOMEM;
+    for (m = 0; m < p->ncombos; m++) {
+        const sg_unit_combo *cb = &p->combos[m];
+        for (q = 0; q < g; q++) {
+            const int j = cb->lv[q];
+            int below = 0, e, side;
+            if (j < 1) continue;
+            for (i = q + 1; i < g; i++) below += cb->lv[i]; /* index bits under dim q's */
+            for (e = 0; e < 1 << cb->sum; e++) {
+                const int ik = (e >> below) & ((1 << j) - 1), hi = e >> (below + j), lw = e & ((1 << below) - 1);
+                sg_unit_node *out = &p->nodes[fill[q][j]++];
+                out->node = (uint16_t)(cb->node + (uint32_t)e);
+                out->pad = 0;
+                for (side = 0; side < 2; side++) {
+                    int pl = 0, pi = parent_of(ik, j, side, &pl), l3[3] = {cb->lv[0], cb->lv[1], cb->lv[2]};
+                    uint16_t at = SG_UNIT_NONE;
+                    if (pi >= 0) {
+                        l3[q] = pl;
+                        at = (uint16_t)(p->combos[id[l3[0]][l3[1]][l3[2]]].node +
+                                        (uint32_t)((((hi << pl) | pi) << below) | lw));
+                    }
+                    if (side == 0) out->left = at;
+                    else out->right = at;
+                }
+            }
+        }
+    }
+    memset(&ctx, 0, sizeof(ctx));
+    memset(lv, 0, sizeof(lv));
+    ctx.L = L;
+    ctx.p = p;
+    ctx.k0 = k0;
+    ctx.g = g;
+    m = 0;
+    for (i = 0; i < L->d; i++)
+        if (i < k0 || i >= k0 + g) dims[m++] = i;
+    enum_levels(L, dims, m, 0, L->n - 1, 0, lv, unit_visit, &ctx);
+    if (ctx.err) return ctx.err;
+    if (p->nunits > 1) qsort(p->units, (size_t)p->nunits, sizeof(sg_unit), unit_cmp);
+    return SG_OK;
+}
+
+int64_t sg_layout_sweep_bytes(const sg_layout *L)
+{
+    int64_t b = 0;
+    int k, g;
+    for (k = 0; k < L->d; k += g > 0 ? g : 1) {
+        g = sg_layout_pass_dims(L, k, 4);
+        if (g > 0) b += (8 * g + 2) * pass_nodes(L, k, g, L->n - 1) + 8 * SG_MAX_LEVELS * SG_MAX_LEVELS * SG_MAX_LEVELS / 8;
+        b += 12 * L->S + 4096; /* chains or units, and subspace offsets */
+    }
+    return b;
+}
+
 /* ---- evaluation (block) layout ------------------------------------------ */
 
 static int lim_of(const sg_layout *L, int k) { return k >= 0 ? L->lim[k] : 0; }

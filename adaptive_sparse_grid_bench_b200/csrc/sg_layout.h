@@ -59,6 +59,67 @@ int sg_layout_chains(const sg_layout *L, int k, sg_chain **chains, int64_t *ncha
                      uint32_t **seg_off, int64_t *nseg);
 
 
+/* ---- passes of several sweeps (hier_fused.cu) ---------------------------
+ * A pass runs the sweeps of dims k0..k0+g-1.  A unit holds the subspaces that
+ * differ only in those dims' levels: 2^sigma cells of a g-dimensional grid of
+ * budget R.  The nodes of that grid are numbered by level sum, so the grid of
+ * a smaller budget is a prefix. */
+typedef struct sg_unit {
+    uint32_t off;  /* first of its subspace offsets, one per combo of sum <= R */
+    uint8_t R;     /* level budget of the pass's dims                          */
+    uint8_t sigma; /* level sum of the other dims                              */
+    uint8_t lo;    /* of those after the pass's dims                           */
+    uint8_t pad;
+} sg_unit;
+typedef struct sg_unit_combo { /* levels of the pass's dims */
+    uint32_t node;             /* first node                */
+    uint8_t lv[3], sum;
+} sg_unit_combo;
+typedef struct sg_unit_node { /* a point that a sweep updates, and its parents */
+    uint16_t node, left, right, pad;
+} sg_unit_node;
+#define SG_UNIT_NONE 0xFFFF
+typedef struct sg_unit_tables {
+    const sg_unit_combo *combos; /* device */
+    const sg_unit_node *nodes;   /* device: per dim q and level j, ordered by level sum */
+    int lmax[3];
+    const uint16_t *combo_of;    /* device: the combo of each node */
+    int ncombo[SG_MAX_LEVELS], nnode[SG_MAX_LEVELS]; /* combos, nodes of sum <= R  */
+    uint32_t first[3][SG_MAX_LEVELS];               /* first entry of (q, j)       */
+    uint16_t count[3][SG_MAX_LEVELS][SG_MAX_LEVELS]; /* entries of (q, j) of sum <= R */
+} sg_unit_tables;
+/* Shared-memory row of a node: its cells, padded against bank conflicts
+ * between the nodes that one 16-byte load scatters to. */
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int sgk_unit_stride(int sigma)
+{
+    return (1 << sigma) + (sigma >= 3 ? 4 : 0);
+}
+#define SG_UNIT_MAX_BYTES (100 * 1024) /* two CTAs per SM at least */
+#define SG_PASS_NODES 10240
+#define SG_PASS3_NODES 1100
+#define SG_PASS1_BYTES (48 * 1024)
+/* The dims a pass from k0 on should run (0: none; the single-dim sweeps do
+ * better), for elements of elem_bytes. */
+int sg_layout_pass_dims(const sg_layout *L, int k0, int elem_bytes);
+/* The pass's tables, all malloc'd (NULL on failure); tables' pointers unset.
+ * max_elems: shared-memory elements of its largest unit. */
+typedef struct sg_pass_host {
+    sg_unit *units;
+    uint32_t *offs;
+    sg_unit_combo *combos;
+    sg_unit_node *nodes;
+    uint16_t *combo_of;
+    int64_t nunits, noffs, ncombos, nnodes, nall, max_elems;
+    sg_unit_tables tables;
+} sg_pass_host;
+int sg_layout_pass(const sg_layout *L, int k0, int g, sg_pass_host *p);
+void sg_layout_pass_free(sg_pass_host *p);
+/* Upper bound of the device bytes of all sweep tables. */
+int64_t sg_layout_sweep_bytes(const sg_layout *L);
+
 /*
  * Evaluation layout ("block layout").  The same surpluses, ordered for the
  * evaluation walk.  Dims 0..d-4 form the prefix; the three innermost dims are

@@ -95,8 +95,16 @@ static void free_device(sg_grid *g)
     dev_free(g, g->d_repack);
     dev_free(g, g->d_rsrc);
     for (k = 0; k < SG_MAX_DIMS; k++) {
+        int f;
         dev_free(g, g->d_chains[k]);
         dev_free(g, g->d_seg[k]);
+        for (f = 0; f < 2; f++) {
+            dev_free(g, g->pass[f][k].units);
+            dev_free(g, g->pass[f][k].offs);
+            dev_free(g, g->pass[f][k].combos);
+            dev_free(g, g->pass[f][k].nodes);
+            dev_free(g, g->pass[f][k].combo_of);
+        }
     }
     dev_free(g, g->d_err);
     dev_free(g, g->d_scratch);
@@ -250,6 +258,104 @@ static void leave(sg_grid *g, int prev)
     if (g->dev >= 0 && g->dev != prev) cudaSetDevice(prev);
 }
 
+static int dev_upload(sg_grid *g, void **p, const void *src, int64_t bytes, cudaStream_t st, const char *what)
+{
+    cudaError_t e;
+    int r = dev_alloc(g, p, bytes, what);
+    if (r != SG_OK || bytes <= 0) return r;
+    /* pageable source: the copy has taken the bytes when the call returns */
+    e = cudaMemcpyAsync(*p, src, (size_t)bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? SG_OK : cuda_fail(e, what);
+}
+
+/* The chain table of dim k (single-dim sweeps). */
+static int build_chains(sg_grid *g, int k, cudaStream_t st)
+{
+    const sg_layout *L = &g->L;
+    sg_chain *ch = NULL;
+    uint32_t *seg = NULL;
+    int64_t nch = 0, nseg = 0, c, cap32 = 0, cap64 = 0;
+    int lmax_max = 0, r;
+    if (g->d_chains[k]) return SG_OK;
+    if ((r = sg_layout_chains(L, k, &ch, &nch, &seg, &nseg)) != SG_OK)
+        return fail(r, "building the sweep tables of dim %d", k);
+    for (c = 0; c < nch; c++) {
+        int j;
+        int64_t e32 = 0, e64 = 0;
+        for (j = 0; j <= ch[c].lmax; j++) {
+            int64_t sz = (int64_t)1 << (ch[c].sigma + j);
+            e32 += sz < 4 ? 4 : sz;
+            e64 += sz < 2 ? 2 : sz;
+        }
+        if (e32 > cap32) cap32 = e32;
+        if (e64 > cap64) cap64 = e64;
+        if (ch[c].lmax > lmax_max) lmax_max = ch[c].lmax;
+    }
+    r = dev_upload(g, (void **)&g->d_seg[k], seg, nseg * 4, st, "sweep segments");
+    if (r == SG_OK)
+        r = dev_upload(g, (void **)&g->d_chains[k], ch, nch * (int64_t)sizeof(sg_chain), st, "sweep chains");
+    free(ch);
+    free(seg);
+    if (r != SG_OK) return r;
+    g->sweep[k].chains = g->d_chains[k];
+    g->sweep[k].seg = g->d_seg[k];
+    g->sweep[k].nchains = nch;
+    g->sweep[k].lmax_max = lmax_max;
+    g->sweep[k].cap32 = cap32;
+    g->sweep[k].cap64 = cap64;
+    return SG_OK;
+}
+
+/* The passes of the current precision (f: 0 FP32, 1 FP64). */
+static int build_passes(sg_grid *g, int f, cudaStream_t st)
+{
+    const sg_layout *L = &g->L;
+    int k, r, n = 0;
+    if (g->npass[f]) return SG_OK;
+    for (k = 0; k < L->d; n++) {
+        sg_pass_state *ps = &g->pass[f][n];
+        sg_pass_host h;
+        const int dims = sg_layout_pass_dims(L, k, f ? 8 : 4);
+        ps->k0 = k;
+        ps->p.g = dims;
+        k += dims ? dims : 1;
+        if (!dims) {
+            if ((r = build_chains(g, ps->k0, st)) != SG_OK) return r;
+            continue;
+        }
+        r = sg_layout_pass(L, ps->k0, dims, &h);
+        if (r != SG_OK) fail(r, "building the sweep tables of dims %d..%d", ps->k0, k - 1);
+        if (r == SG_OK) r = dev_upload(g, (void **)&ps->units, h.units, h.nunits * (int64_t)sizeof(sg_unit), st, "sweep units");
+        if (r == SG_OK) r = dev_upload(g, (void **)&ps->offs, h.offs, h.noffs * 4, st, "unit offsets");
+        if (r == SG_OK) r = dev_upload(g, (void **)&ps->combos, h.combos, h.ncombos * (int64_t)sizeof(sg_unit_combo), st, "unit levels");
+        if (r == SG_OK) r = dev_upload(g, (void **)&ps->nodes, h.nodes, h.nnodes * (int64_t)sizeof(sg_unit_node), st, "unit nodes");
+        if (r == SG_OK) r = dev_upload(g, (void **)&ps->combo_of, h.combo_of, h.nall * 2, st, "unit node levels");
+        ps->p.units = ps->units;
+        ps->p.offs = ps->offs;
+        ps->p.nunits = h.nunits;
+        ps->p.max_elems = h.max_elems;
+        ps->p.tables = h.tables;
+        ps->p.tables.combos = ps->combos;
+        ps->p.tables.nodes = ps->nodes;
+        ps->p.tables.combo_of = ps->combo_of;
+        sg_layout_pass_free(&h);
+        if (r != SG_OK) return r;
+    }
+    g->npass[f] = n;
+    return SG_OK;
+}
+
+/* The sweep tables that the handle's options call for. */
+static int build_sweeps(sg_grid *g, cudaStream_t st)
+{
+    int k, r = SG_OK;
+    if (g->opt[SG_OPT_HIER_KERNEL] == 2 || g->opt[SG_OPT_TEST_WAIT] > 0)
+        for (k = 0; k < g->L.d && r == SG_OK; k++) r = build_chains(g, k, st);
+    else
+        r = build_passes(g, g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64, st);
+    return r;
+}
+
 /* Allocates the handle's device state and uploads its tables.  The clears
  * and uploads go on `st` (the stream of the call that needs the state, never
  * the legacy default stream, so a serving loop's streams do not wait on
@@ -261,7 +367,7 @@ static int materialize(sg_grid *g, cudaStream_t st)
     sg_repack *rp = NULL;
     uint32_t *rs = NULL, *st_tab = NULL;
     int64_t words;
-    int k, r;
+    int r;
     cudaError_t ce;
     if (g->dev >= 0) return SG_OK;
     CU((cudaError_t)sgk_eval_setup(), "evaluation kernel set-up");
@@ -310,45 +416,7 @@ static int materialize(sg_grid *g, cudaStream_t st)
         st_tab = NULL;
     }
     g->eval_dirty = 1;
-    for (k = 0; k < L->d; k++) {
-        sg_chain *ch = NULL;
-        uint32_t *seg = NULL;
-        int64_t nch = 0, nseg = 0, c, cap32 = 0, cap64 = 0;
-        int lmax_max = 0;
-        if ((r = sg_layout_chains(L, k, &ch, &nch, &seg, &nseg)) != SG_OK) {
-            fail(r, "building the sweep tables of dim %d", k);
-            goto bad;
-        }
-        for (c = 0; c < nch; c++) {
-            int j;
-            int64_t e32 = 0, e64 = 0;
-            for (j = 0; j <= ch[c].lmax; j++) {
-                int64_t sz = (int64_t)1 << (ch[c].sigma + j);
-                e32 += sz < 4 ? 4 : sz;
-                e64 += sz < 2 ? 2 : sz;
-            }
-            if (e32 > cap32) cap32 = e32;
-            if (e64 > cap64) cap64 = e64;
-            if (ch[c].lmax > lmax_max) lmax_max = ch[c].lmax;
-        }
-        r = dev_alloc(g, (void **)&g->d_chains[k], nch * (int64_t)sizeof(sg_chain), "sweep chains");
-        if (r == SG_OK) r = dev_alloc(g, (void **)&g->d_seg[k], nseg * 4, "sweep segments");
-        if (r == SG_OK && nch > 0) {
-            cudaError_t e =
-                cudaMemcpyAsync(g->d_chains[k], ch, (size_t)nch * sizeof(sg_chain), cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_seg[k], seg, (size_t)nseg * 4, cudaMemcpyHostToDevice, st);
-            if (e != cudaSuccess) r = cuda_fail(e, "uploading sweep tables");
-        }
-        free(ch);
-        free(seg);
-        if (r != SG_OK) goto bad;
-        g->sweep[k].chains = g->d_chains[k];
-        g->sweep[k].seg = g->d_seg[k];
-        g->sweep[k].nchains = nch;
-        g->sweep[k].lmax_max = lmax_max;
-        g->sweep[k].cap32 = cap32;
-        g->sweep[k].cap64 = cap64;
-    }
+    if ((r = build_sweeps(g, st)) != SG_OK) goto bad;
     if ((ce = cudaStreamSynchronize(st)) != cudaSuccess) {
         r = cuda_fail(ce, "uploading the grid tables");
         goto bad;
@@ -362,6 +430,8 @@ bad:
     free_device(g);
     memset(g->d_chains, 0, sizeof(g->d_chains));
     memset(g->d_seg, 0, sizeof(g->d_seg));
+    memset(g->pass, 0, sizeof(g->pass));
+    memset(g->npass, 0, sizeof(g->npass));
     g->d_alpha = NULL;
     g->d_work = NULL;
     g->d_blk = NULL;
@@ -490,38 +560,52 @@ SG_API int sg_timings(sg_grid *g, double *ms)
     return r;
 }
 
+/* All sweeps of the stored values in place: passes of several dims, and
+ * single-dim sweeps where a pass does not apply or the options ask for them. */
+static int sweeps_on(sg_grid *g, int f64, cudaStream_t st)
+{
+    const int kern = (int)g->opt[SG_OPT_HIER_KERNEL], stall = (int)g->opt[SG_OPT_TEST_WAIT];
+    int i, k, e;
+    if (kern != 2 && stall <= 0) {
+        for (i = 0; i < g->npass[f64]; i++) {
+            const sg_pass_state *ps = &g->pass[f64][i];
+            if (ps->p.g)
+                e = f64 ? sgk_sweep_fused_f64(g->d_work, &ps->p, st) : sgk_sweep_fused_f32(g->d_alpha, &ps->p, st);
+            else if (sgk_chain_smem_bytes(f64 ? g->sweep[ps->k0].cap64 : g->sweep[ps->k0].cap32, f64 ? 8 : 4) >= 0)
+                e = f64 ? sgk_sweep_chains_f64(g->d_work, &g->sweep[ps->k0], g->d_err, st)
+                        : sgk_sweep_chains_f32(g->d_alpha, &g->sweep[ps->k0], g->d_err, st);
+            else
+                e = f64 ? sgk_sweep_gather_f64(g->d_work, &g->sweep[ps->k0], st)
+                        : sgk_sweep_gather_f32(g->d_alpha, &g->sweep[ps->k0], st);
+            if (e != cudaSuccess) return cuda_fail((cudaError_t)e, "sweep");
+        }
+        return SG_OK;
+    }
+    for (k = 0; k < g->L.d; k++) {
+        const int fits = sgk_chain_smem_bytes(f64 ? g->sweep[k].cap64 : g->sweep[k].cap32, f64 ? 8 : 4) >= 0;
+        if (!f64 && stall > 0 && fits)
+            e = sgk_sweep_chains_stall_f32(g->d_alpha, &g->sweep[k], g->d_err, (int64_t)stall << 20, st);
+        else if (kern != 2 && fits)
+            e = f64 ? sgk_sweep_chains_f64(g->d_work, &g->sweep[k], g->d_err, st)
+                    : sgk_sweep_chains_f32(g->d_alpha, &g->sweep[k], g->d_err, st);
+        else
+            e = f64 ? sgk_sweep_gather_f64(g->d_work, &g->sweep[k], st)
+                    : sgk_sweep_gather_f32(g->d_alpha, &g->sweep[k], st);
+        if (e != cudaSuccess) return cuda_fail((cudaError_t)e, "sweep");
+    }
+    return SG_OK;
+}
+
 static int hierarchize_on(sg_grid *g, cudaStream_t st)
 {
     const sg_layout *L = &g->L;
-    const int prec = (int)g->opt[SG_OPT_HIER_PRECISION];
-    const int kern = (int)g->opt[SG_OPT_HIER_KERNEL];
-    int k, e;
-    if (prec == SG_HIER_FP64) {
-        if (!g->d_work) {
-            int r = dev_alloc(g, (void **)&g->d_work, L->Npad * 8, "FP64 working grid");
-            if (r != SG_OK) return r;
-        }
-        if ((e = sgk_widen(g->d_alpha, g->d_work, L->Npad, st)) != cudaSuccess)
-            return cuda_fail((cudaError_t)e, "widen");
-        for (k = 0; k < L->d; k++) {
-            const int fits = sgk_chain_smem_bytes(g->sweep[k].cap64, 8) >= 0;
-            e = (kern != 2 && fits) ? sgk_sweep_chains_f64(g->d_work, &g->sweep[k], g->d_err, st)
-                                    : sgk_sweep_gather_f64(g->d_work, &g->sweep[k], st);
-            if (e != cudaSuccess) return cuda_fail((cudaError_t)e, "FP64 sweep");
-        }
-        if ((e = sgk_narrow(g->d_work, g->d_alpha, L->Npad, st)) != cudaSuccess)
-            return cuda_fail((cudaError_t)e, "narrow");
-        return SG_OK;
-    }
-    for (k = 0; k < L->d; k++) {
-        const int fits = sgk_chain_smem_bytes(g->sweep[k].cap32, 4) >= 0;
-        if (g->opt[SG_OPT_TEST_WAIT] > 0 && fits)
-            e = sgk_sweep_chains_stall_f32(g->d_alpha, &g->sweep[k], g->d_err, g->opt[SG_OPT_TEST_WAIT] << 20, st);
-        else
-            e = (kern != 2 && fits) ? sgk_sweep_chains_f32(g->d_alpha, &g->sweep[k], g->d_err, st)
-                                    : sgk_sweep_gather_f32(g->d_alpha, &g->sweep[k], st);
-        if (e != cudaSuccess) return cuda_fail((cudaError_t)e, "FP32 sweep");
-    }
+    int e, r = build_sweeps(g, st); /* built with the values, unless the options changed since */
+    if (r != SG_OK) return r;
+    if (g->opt[SG_OPT_HIER_PRECISION] != SG_HIER_FP64) return sweeps_on(g, 0, st);
+    if (!g->d_work && (r = dev_alloc(g, (void **)&g->d_work, L->Npad * 8, "FP64 working grid")) != SG_OK) return r;
+    if ((e = sgk_widen(g->d_alpha, g->d_work, L->Npad, st)) != cudaSuccess) return cuda_fail((cudaError_t)e, "widen");
+    if ((r = sweeps_on(g, 1, st)) != SG_OK) return r;
+    if ((e = sgk_narrow(g->d_work, g->d_alpha, L->Npad, st)) != cudaSuccess) return cuda_fail((cudaError_t)e, "narrow");
     return SG_OK;
 }
 
@@ -629,10 +713,16 @@ SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_
     if (r == SG_OK) g->opt[SG_OPT_EVAL_BLOCKING] = bi + 1;
     /* hierarchization: shared-memory chains (where they fit) vs gather; the
      * values are saved first and restored at the end */
-    for (k = 0; k < g->L.d; k++)
-        if (sgk_chain_smem_bytes(g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64 ? g->sweep[k].cap64 : g->sweep[k].cap32,
-                                 g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64 ? 8 : 4) >= 0)
-            chains_apply = 1;
+    if (r == SG_OK) {
+        const int f = g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64;
+        g->opt[SG_OPT_HIER_KERNEL] = 1;
+        r = build_sweeps(g, ta.st);
+        for (k = 0; r == SG_OK && k < g->npass[f]; k++) {
+            const sg_pass_state *ps = &g->pass[f][k];
+            if (ps->p.g || sgk_chain_smem_bytes(f ? g->sweep[ps->k0].cap64 : g->sweep[ps->k0].cap32, f ? 8 : 4) >= 0)
+                chains_apply = 1;
+        }
+    }
     if (r == SG_OK) r = dev_alloc(g, (void **)&saved, g->L.Npad * 4, "sg_autotune saved values");
     if (r == SG_OK) {
         cudaError_t e = cudaMemcpyAsync(saved, g->d_alpha, (size_t)g->L.Npad * 4, cudaMemcpyDeviceToDevice, ta.st);
@@ -998,6 +1088,16 @@ SG_API int sg_set_option(sg_grid *g, int option, int64_t value)
         return fail(SG_ERR_ARG, "unknown option %d", option);
     }
     g->opt[option] = value;
+    if (g->dev >= 0 && (option == SG_OPT_HIER_PRECISION || option == SG_OPT_HIER_KERNEL || option == SG_OPT_TEST_WAIT)) {
+        /* the sweep tables of the new setting, here rather than in a
+         * hierarchization that may be under stream capture */
+        int prev, r = enter(g, &prev);
+        if (r != SG_OK) return r;
+        r = build_sweeps(g, 0);
+        if (r == SG_OK && cudaStreamSynchronize(0) != cudaSuccess) r = cuda_fail(cudaGetLastError(), "uploading sweep tables");
+        leave(g, prev);
+        return r;
+    }
     return SG_OK;
 }
 
