@@ -88,55 +88,93 @@ struct FnParams {
     double p[SG_MAX_FN_PARAMS];
 };
 
-/* One thread per device element; padding elements between groups are set
- * to 0.  x_k = (2 i_k + 1) / 2^(l_k+1) is exact in FP32 and FP64. */
-__global__ void k_sample(const Tables T, const FnParams F, float *__restrict__ alpha, int64_t npad)
+/* f at the grid points, four consecutive elements of the layout per thread.  In
+ * a group of level sum s >= 2 they lie in one subspace, so its level vector is
+ * found once for the four (it was most of the time, with a double division per
+ * coordinate: x_k = (2 i_k + 1) / 2^(l_k+1) is exact, as a product with a power
+ * of two too).  d = 6, n = 12 (limits 9, 8), N = 13.3 M, Gaussian bump: see
+ * sgk_sample.  Padding between groups is set to 0. */
+struct SampleTables {
+    int d, n;
+    uint32_t dp[SG_MAX_DIMS][SG_MAX_LEVELS];
+    uint32_t size[SG_MAX_LEVELS];       /* values of group s         */
+    uint32_t start[SG_MAX_LEVELS + 1];  /* first place of group s    */
+};
+
+template <int FN>
+__device__ __forceinline__ void sample_term(double &acc, double x, int k, const FnParams &F)
 {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < npad;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        int s = 0;
-        while (s < T.n && j >= T.plidx[s + 1]) ++s;
-        if (s >= T.n) {
-            alpha[j] = 0.0f;
-            continue;
-        }
-        const int64_t local = j - T.plidx[s];
-        const int64_t gsize = (T.lidx[s + 1] - T.lidx[s]);
-        if (local >= gsize) {
-            alpha[j] = 0.0f;
-            continue;
-        }
-        int64_t pos = local >> s, rest = local & (((int64_t)1 << s) - 1);
-        int lvl[SG_MAX_DIMS];
-        int ss = s;
-        for (int i = T.d - 1; i >= 1; --i) {
-            int level = 0;
-            while (pos >= T.dp[i - 1][ss - level]) {
-                pos -= T.dp[i - 1][ss - level];
-                ++level;
+    if constexpr (FN == SG_FN_REFERENCE) acc += x * x * (1.0 - x) * (1.0 - x);
+    else if constexpr (FN == SG_FN_PROD4) acc *= 4.0 * x * (1.0 - x);
+    else if constexpr (FN == SG_FN_GAUSS) acc += x * x;
+    else if constexpr (FN == SG_FN_BUMP) acc += (x - F.p[0]) * (x - F.p[0]);
+    else acc *= F.p[3 * k] + F.p[3 * k + 1] * x + F.p[3 * k + 2] * x * x;
+}
+
+/* values q .. q + P - 1 of group s, all in one subspace */
+template <int FN, int P>
+__device__ __forceinline__ void sample_points(const SampleTables &T, const FnParams &F, int s, uint32_t q, float (&out)[P])
+{
+    uint32_t pos = q >> s, rest = q & ((1u << s) - 1u);
+    double acc[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) acc[p] = (FN == SG_FN_PROD4 || FN == SG_FN_QUAD) ? 1.0 : 0.0;
+    /* the levels come out last dim first, which is the order of the index
+     * bits and of the sums */
+    int left = s, shift = 0;
+    for (int k = T.d - 1; k >= 0; --k) {
+        int l = 0;
+        if (k >= 1) {
+            uint32_t c = T.dp[k - 1][left];
+            while (pos >= c) {
+                pos -= c;
+                ++l;
+                c = T.dp[k - 1][left - l];
             }
-            lvl[i] = level;
-            ss -= level;
+        } else {
+            l = left;
         }
-        lvl[0] = ss;
-        double acc = (F.fn == SG_FN_PROD4 || F.fn == SG_FN_QUAD) ? 1.0 : 0.0;
-        for (int k = T.d - 1; k >= 0; --k) {
-            const int64_t ik = rest & (((int64_t)1 << lvl[k]) - 1);
-            rest >>= lvl[k];
-            const double x = (double)(2 * ik + 1) / (double)((int64_t)2 << lvl[k]);
-            switch (F.fn) {
-            case SG_FN_REFERENCE: acc += x * x * (1.0 - x) * (1.0 - x); break;
-            case SG_FN_PROD4: acc *= 4.0 * x * (1.0 - x); break;
-            case SG_FN_GAUSS: acc += x * x; break;
-            case SG_FN_BUMP: acc += (x - F.p[0]) * (x - F.p[0]); break;
-            case SG_FN_QUAD: acc *= F.p[3 * k] + F.p[3 * k + 1] * x + F.p[3 * k + 2] * x * x; break;
-            default: break;
+        left -= l;
+        const double scale = __hiloint2double((1022 - l) << 20, 0); /* 2^-(l+1) */
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const uint32_t ik = ((rest + p) >> shift) & ((1u << l) - 1u);
+            sample_term<FN>(acc[p], (double)(2 * ik + 1) * scale, k, F);
+        }
+        shift += l;
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        double v = acc[p];
+        if (FN == SG_FN_GAUSS) v = exp(-acc[p]);
+        if (FN == SG_FN_BUMP) v = exp(-F.p[1] * acc[p]);
+        out[p] = __double2float_rn(v);
+    }
+}
+
+template <int FN>
+__global__ void __launch_bounds__(256) k_sample(const SampleTables T, const FnParams F, float *__restrict__ alpha,
+                                                int64_t npad)
+{
+    for (int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; j < npad;
+         j += (int64_t)gridDim.x * blockDim.x * 4) {
+        int s = T.n - 1;
+        while (j < T.start[s]) --s;
+        const uint32_t q = (uint32_t)j - T.start[s], size = T.size[s];
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (s >= 2) {
+            if (q < size) sample_points<FN, 4>(T, F, s, q, v);
+        } else {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                float one[1];
+                if (q + p < size) {
+                    sample_points<FN, 1>(T, F, s, q + p, one);
+                    v[p] = one[0];
+                }
             }
         }
-        double v = acc;
-        if (F.fn == SG_FN_GAUSS) v = exp(-acc);
-        if (F.fn == SG_FN_BUMP) v = exp(-F.p[1] * acc);
-        alpha[j] = __double2float_rn(v);
+        *reinterpret_cast<float4 *>(alpha + j) = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
 
@@ -188,9 +226,26 @@ int sgk_sample(const sg_layout *L, int fn, const double *params, int nparams, fl
     F.np = nparams;
     for (int i = 0; i < SG_MAX_FN_PARAMS; ++i) F.p[i] = i < nparams ? params[i] : 0.0;
     if (L->Npad <= 0) return cudaSuccess;
-    int64_t g = (L->Npad + 255) / 256;
-    if (g > 148 * 32) g = 148 * 32;
-    k_sample<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(make_tables(L), F, alpha, L->Npad);
+    SampleTables T;
+    T.d = L->d;
+    T.n = L->n;
+    for (int i = 0; i < SG_MAX_DIMS; ++i)
+        for (int q = 0; q < SG_MAX_LEVELS; ++q) T.dp[i][q] = i < L->d && q < L->n ? (uint32_t)L->dp[i][q] : 0;
+    for (int q = 0; q <= SG_MAX_LEVELS; ++q) {
+        if (q < SG_MAX_LEVELS) T.size[q] = q < L->n ? (uint32_t)(L->lidx[q + 1] - L->lidx[q]) : 0;
+        T.start[q] = (uint32_t)L->plidx[q < L->n ? q : L->n];
+    }
+    int64_t g = (L->Npad / 4 + 255) / 256;
+    if (g > 148 * 8) g = 148 * 8;
+    cudaStream_t st = (cudaStream_t)stream;
+    switch (fn) {
+    case SG_FN_REFERENCE: k_sample<SG_FN_REFERENCE><<<(unsigned)g, 256, 0, st>>>(T, F, alpha, L->Npad); break;
+    case SG_FN_PROD4: k_sample<SG_FN_PROD4><<<(unsigned)g, 256, 0, st>>>(T, F, alpha, L->Npad); break;
+    case SG_FN_GAUSS: k_sample<SG_FN_GAUSS><<<(unsigned)g, 256, 0, st>>>(T, F, alpha, L->Npad); break;
+    case SG_FN_BUMP: k_sample<SG_FN_BUMP><<<(unsigned)g, 256, 0, st>>>(T, F, alpha, L->Npad); break;
+    case SG_FN_QUAD: k_sample<SG_FN_QUAD><<<(unsigned)g, 256, 0, st>>>(T, F, alpha, L->Npad); break;
+    default: return cudaErrorInvalidValue;
+    }
     sgk_count(1);
     return cudaGetLastError();
 }
