@@ -22,7 +22,6 @@
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kMaxUpdated = 512; /* updated points per chain for n <= 9: < 2^9 */
 constexpr int kPerLane = kMaxUpdated / 32;
 
@@ -59,8 +58,11 @@ __device__ __forceinline__ T point_update(const T *buf, const uint32_t *__restri
     return upd(buf[w], lft, rgt);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_hier_smem(float *__restrict__ a, const sg_smem_grid *__restrict__ grids,
+/* NT threads: the grid is one CTA's work, so larger grids get more warps (the
+ * batch of 96 mixed grids, whose 57 small ones leave most SMs idle: 1109 us of
+ * kernels with 256 threads for all; see launch). */
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) k_hier_smem(float *__restrict__ a, const sg_smem_grid *__restrict__ grids,
                                                        const sg_chain *__restrict__ chains,
                                                        const uint32_t *__restrict__ seg)
 {
@@ -68,11 +70,11 @@ __global__ void __launch_bounds__(kThreads) k_hier_smem(float *__restrict__ a, c
     T *buf = reinterpret_cast<T *>(smem_raw);
     const sg_smem_grid g = grids[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int nwarps = kThreads / 32;
+    constexpr int nwarps = NT / 32;
     float *src = a + g.base;
 
     /* load (npad and base are multiples of 32: 16-byte vector loads) */
-    for (int i = tid * 4; i < (int)g.npad; i += kThreads * 4) {
+    for (int i = tid * 4; i < (int)g.npad; i += NT * 4) {
         const float4 v = *reinterpret_cast<const float4 *>(src + i);
         buf[i] = (T)v.x;
         buf[i + 1] = (T)v.y;
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(kThreads) k_hier_smem(float *__restrict__ a, c
         __syncthreads();
     }
 
-    for (int i = tid * 4; i < (int)g.npad; i += kThreads * 4) {
+    for (int i = tid * 4; i < (int)g.npad; i += NT * 4) {
         float4 v;
         if constexpr (sizeof(T) == 8) {
             v = make_float4(__double2float_rn(buf[i]), __double2float_rn(buf[i + 1]),
@@ -118,6 +120,17 @@ __global__ void __launch_bounds__(kThreads) k_hier_smem(float *__restrict__ a, c
     }
 }
 
+template <typename T, int NT>
+int launch_nt(float *a, const sg_smem_grid *grids, int ngrids, const sg_chain *chains, const uint32_t *seg, size_t smem,
+              void *stream)
+{
+    cudaError_t e = cudaFuncSetAttribute(k_hier_smem<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_hier_smem<T, NT><<<ngrids, NT, smem, (cudaStream_t)stream>>>(a, grids, chains, seg);
+    sgk_count(1);
+    return cudaGetLastError();
+}
+
 template <typename T>
 int launch(float *a, const sg_smem_grid *grids, int ngrids, const sg_chain *chains, const uint32_t *seg,
            int max_npad, void *stream)
@@ -125,11 +138,9 @@ int launch(float *a, const sg_smem_grid *grids, int ngrids, const sg_chain *chai
     if (ngrids <= 0) return cudaSuccess;
     const size_t smem = (size_t)max_npad * sizeof(T);
     if (smem > SG_SMEM_GRID_MAX_BYTES) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_hier_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_hier_smem<T><<<ngrids, kThreads, smem, (cudaStream_t)stream>>>(a, grids, chains, seg);
-    sgk_count(1);
-    return cudaGetLastError();
+    if (max_npad <= 1024) return launch_nt<T, 256>(a, grids, ngrids, chains, seg, smem, stream);
+    if (max_npad <= 4096) return launch_nt<T, 512>(a, grids, ngrids, chains, seg, smem, stream);
+    return launch_nt<T, 1024>(a, grids, ngrids, chains, seg, smem, stream);
 }
 
 } // namespace
