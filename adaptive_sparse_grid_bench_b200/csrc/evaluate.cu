@@ -37,6 +37,9 @@ __device__ __forceinline__ void kahan(float &s, float &c, float v)
 __device__ __forceinline__ float combine(const float *__restrict__ src, int64_t m, int nseg, int nparts, int emit)
 {
     float s = 0.0f, c = 0.0f;
+    /* a point with a NaN coordinate: the NaN its warps wrote, not an
+     * arithmetic one */
+    if (__float_as_uint(src[0]) == 0x7fc00000u) return src[0];
     if (emit == SG_EMIT_PARTS) {
         for (int k = 0; k < nparts; ++k) kahan(s, c, src[k * m]);
         return __fsub_rn(s, c);

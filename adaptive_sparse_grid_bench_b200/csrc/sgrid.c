@@ -813,7 +813,9 @@ static void grid_plan(const sg_grid *g, sg_eval_plan *p)
  * whole-sum launch would fill less than 3/4 of its rounds of resident warps (16
  * per SM, 64 points each) the segments of a sum go to several warps.  (The
  * kernel that can share is about a quarter slower per point than the one that
- * cannot.)  d = 10, n = 10: 7.35 -> 0.17 ms for 1,000 points, 6.05 -> 3.3 ms for
+ * cannot; above 12 dims, where its walk down to each segment is long, twice as
+ * slow, so there only below a quarter: d = 16, n = 5, 65,536 points 1.2 ms whole,
+ * 2.1 ms shared.)  d = 10, n = 10: 7.35 -> 0.17 ms for 1,000 points, 6.05 -> 3.3 ms for
  * 65,536; 2^20 points share at a loss (35.3 -> 42.9 ms).  Returns the floats of
  * part_out (0: whole sums).  No choice changes a result. */
 static int64_t plan_shares(const sg_grid *g, int64_t m, sg_eval_plan *p)
@@ -822,7 +824,7 @@ static int64_t plan_shares(const sg_grid *g, int64_t m, sg_eval_plan *p)
     int64_t want, floats;
     /* a pool's grids take no scratch beyond the sort's */
     if (p->nseg < SG_SHARE_MIN_SEGS || g->alloc) return 0;
-    if (4 * groups >= 3 * ((groups + room - 1) / room * room)) return 0;
+    if (4 * groups >= (p->d <= 12 ? 3 : 1) * ((groups + room - 1) / room * room)) return 0;
     want = (SG_SHARE_ROUNDS * room + groups - 1) / groups;
     if (want <= p->nparts) {
         p->nshare = p->nparts;

@@ -933,7 +933,7 @@ static int batch_shares(const sg_layout *L, int64_t ctas)
 {
     const int nseg = sg_layout_segs(L), parts = sg_layout_parts(L);
     int64_t n;
-    if (nseg <= 1 || ctas >= SG_BATCH_SHARE_CTAS) return 1;
+    if (nseg <= 1 || ctas >= (L->d <= 12 ? SG_BATCH_SHARE_CTAS : SG_BATCH_SHARE_CTAS / 4)) return 1;
     if (parts > 1) return parts;
     n = L->S / SG_BATCH_SHARE_CHAIN;
     if (n > nseg) n = nseg;
