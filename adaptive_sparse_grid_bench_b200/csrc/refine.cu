@@ -47,22 +47,47 @@ __global__ void __launch_bounds__(256) k_subspace_maxabs(MaxAbsTables T, const f
                     v[t] = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
                 }
             }
-            if (s >= 7) {
+            if (s >= 6) {
+                // A NaN counts where it fills a run of 32 values: the maximum
+                // inside a run passes NaN over, the one over runs compares bit
+                // patterns, which put NaN above infinity.  Without NaN (one
+                // vote per chunk) both are the same maximum.
+                bool nan = false;
+                unsigned u[kSteps];
+#pragma unroll
+                for (int t = 0; t < kSteps; ++t) nan |= v[t] != v[t];
+                if (__any_sync(0xffffffffu, nan)) {
+#pragma unroll
+                    for (int t = 0; t < kSteps; ++t)
+                        for (int off = 1; off < 8; off <<= 1)
+                            v[t] = fmaxf(v[t], __shfl_xor_sync(0xffffffffu, v[t], off));
+                }
+#pragma unroll
+                for (int t = 0; t < kSteps; ++t) u[t] = __float_as_uint(v[t]); // non-negative: ordered like the floats
+                if (s == 6) {
+#pragma unroll
+                    for (int t = 0; t < kSteps; ++t) {
+                        unsigned m = u[t];
+                        for (int off = 1; off < 16; off <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
+                        const int64_t e = first + t * 128 + lane * 4;
+                        if (e < len && (lane & 15) == 0) o[e >> 6] = m;
+                    }
+                    continue;
+                }
                 // 2^(s-7) steps per subspace
                 const int per = s >= 10 ? kSteps : 1 << (s - 7);
-                float m = 0.f;
+                unsigned m = 0;
 #pragma unroll
                 for (int t = 0; t < kSteps; ++t) {
-                    m = fmaxf(m, v[t]);
+                    m = max(m, u[t]);
                     if ((t + 1) % per) continue;
-                    for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+                    for (int off = 16; off; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
                     const int64_t e = first + (int64_t)(t + 1 - per) * 128;
                     if (lane == 0 && e < len) {
-                        // non-negative floats order like their bit patterns
-                        if (s > 10) atomicMax(o + (e >> s), __float_as_uint(m));
-                        else o[e >> s] = __float_as_uint(m);
+                        if (s > 10) atomicMax(o + (e >> s), m);
+                        else o[e >> s] = m;
                     }
-                    m = 0.f;
+                    m = 0;
                 }
             } else {
                 // 2^(s-2) lanes per subspace

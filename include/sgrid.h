@@ -201,7 +201,9 @@ int sg_sample_function(sg_grid *grid, int fn, const double *params, int num_para
  * Levels are 0-based as in the reference. */
 /* maxabs[q] = max |value| over the points of subspace q (subspaces in
  * compact order: level sum s ascending, sg_idx2l positions inside a group);
- * S floats.  Runs on the legacy default stream and waits for it. */
+ * S floats.  NaN values are passed over, except that an aligned run of 32 NaN
+ * (a whole subspace where that is smaller) makes its subspace's maximum NaN.
+ * Runs on the legacy default stream and waits for it. */
 int sg_subspace_maxabs(sg_grid *grid, float *maxabs);
 /* One step: a subspace is active if maxabs > tol; every child l + e_k with
  * l_k < max_level of an active subspace must be in the next grid, which is
