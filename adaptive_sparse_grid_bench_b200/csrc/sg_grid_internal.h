@@ -57,6 +57,7 @@ struct sg_grid {
     int64_t dev_bytes;
     cudaEvent_t ev[SG_NUM_PHASES][2]; /* profiling: start/stop per phase */
     int ev_used[SG_NUM_PHASES];
+    cudaMemPool_t sums_pool; /* the device's pool of segment sums, once used  */
     uint32_t *d_sums;    /* segment table of the sums (sg_layout.h), NULL: one segment */
     sg_dev_alloc_fn alloc; /* NULL: cudaMalloc/cudaFree */
     sg_dev_free_fn free_fn;

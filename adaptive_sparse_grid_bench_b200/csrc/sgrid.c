@@ -6,6 +6,7 @@
  * unusable GPU is reported as SG_ERR_CUDA.
  */
 #include <cuda_runtime_api.h>
+#include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -78,6 +79,89 @@ static void dev_free(sg_grid *g, void *p)
     else cudaFree(p);
 }
 
+/* ---- memory of shared sums ------------------------------------------------ */
+
+#define SG_SHARE_FLOATS ((int64_t)1 << 25) /* largest buffer of segment sums */
+#define SG_POOL_DEVICES 64
+
+/* The segment sums of an evaluation live from its first kernel to its last, on
+ * the caller's stream, and evaluations of one handle may overlap on several
+ * streams, so each takes its own from a stream-ordered pool: 3 us a call, where
+ * growing one buffer took a cudaFree and a cudaMalloc (650 us and a device
+ * synchronization), and a smaller call after a larger one does not free what a
+ * captured evaluation still names.  One pool per device for all handles; it
+ * keeps up to one largest buffer while a handle uses it and gives everything
+ * back with the last one.  Streams never wait for one another to reuse memory. */
+static pthread_mutex_t g_pool_mu = PTHREAD_MUTEX_INITIALIZER;
+static struct {
+    cudaMemPool_t pool;
+    int users;
+} g_pools[SG_POOL_DEVICES];
+
+static void pool_keep(cudaMemPool_t pool, uint64_t bytes)
+{
+    (void)cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes);
+}
+
+static cudaMemPool_t pool_join(int dev)
+{
+    cudaMemPool_t pool = NULL;
+    if (dev >= SG_POOL_DEVICES) return NULL;
+    pthread_mutex_lock(&g_pool_mu);
+    if (!g_pools[dev].pool) {
+        struct cudaMemPoolProps props;
+        int off = 0;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+            (void)cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+            g_pools[dev].pool = pool;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    pool = g_pools[dev].pool;
+    if (pool && g_pools[dev].users++ == 0) pool_keep(pool, 4 * SG_SHARE_FLOATS);
+    pthread_mutex_unlock(&g_pool_mu);
+    return pool;
+}
+
+static void pool_leave(int dev)
+{
+    pthread_mutex_lock(&g_pool_mu);
+    if (--g_pools[dev].users == 0) {
+        pool_keep(g_pools[dev].pool, 0);
+        cudaMemPoolTrimTo(g_pools[dev].pool, 0);
+    }
+    pthread_mutex_unlock(&g_pool_mu);
+}
+
+/* Room for one evaluation's segment sums on st, NULL where there is none (whole
+ * sums need none): out of memory, or st is capturing, where the memory would
+ * have to outlive the call. */
+static float *sums_alloc(sg_grid *g, int64_t floats, cudaStream_t st)
+{
+    enum cudaStreamCaptureStatus cs;
+    enum cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    void *p = NULL;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return NULL;
+    }
+    /* another stream of the process may be capturing: allocating here does not
+     * concern it */
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!g->sums_pool) g->sums_pool = pool_join(g->dev);
+    if (g->sums_pool && cudaMallocFromPoolAsync(&p, (size_t)floats * 4, g->sums_pool, st) != cudaSuccess) {
+        cudaGetLastError();
+        p = NULL;
+    }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return (float *)p;
+}
+
 static void free_device(sg_grid *g)
 {
     int k;
@@ -110,6 +194,8 @@ static void free_device(sg_grid *g)
     dev_free(g, g->d_scratch);
     dev_free(g, g->d_io);
     dev_free(g, g->d_sums);
+    if (g->sums_pool) pool_leave(g->dev);
+    g->sums_pool = NULL;
 }
 
 int sg_create_with_allocator(int d, int n, const int *limits, sg_dev_alloc_fn alloc, sg_dev_free_fn free_fn,
@@ -804,7 +890,6 @@ static void grid_plan(const sg_grid *g, sg_eval_plan *p)
 
 #define SG_SHARE_ROUNDS 3                  /* resident warps' worth of warps to aim for      */
 #define SG_SHARE_MIN_SEGS 4                /* fewer segments: adding them up costs more     */
-#define SG_SHARE_FLOATS ((int64_t)1 << 25) /* largest buffer of segment sums                */
 #define SG_SORT_ROWS ((int64_t)3 << 24)    /* points x rows from which ordering pays        */
 #define SG_SORT_BYTES (192 * 1024)         /* block layouts up to an L1 need no ordering    */
 
@@ -851,22 +936,28 @@ static int plan_sort(const sg_grid *g, int64_t m)
     return g->opt[SG_OPT_EVAL_SORT] && m * g->L.nrows >= SG_SORT_ROWS && g->L.Nblk * 4 > SG_SORT_BYTES;
 }
 
-/* The evaluation launches, with scratch for the sort (sort != 0) followed by
- * the segment sums. */
-typedef struct eval_scratch {
-    int64_t sort_b, coords_b, perm_b, part_b; /* bytes of each region */
-} eval_scratch;
+/* The ordering's scratch regions. */
+typedef struct sort_scratch {
+    int64_t sort_b, coords_b, perm_b; /* bytes of each */
+} sort_scratch;
 
-static int64_t scratch_plan(int64_t m, int d, int sort, int64_t part_floats, eval_scratch *s)
+static int64_t scratch_plan(int64_t m, int d, int sort, sort_scratch *s)
 {
     s->sort_b = sort ? (sgk_sort_scratch_bytes(m, d) + 255) & ~(int64_t)255 : 0;
     s->coords_b = sort ? (m * d * 4 + 255) & ~(int64_t)255 : 0;
     s->perm_b = sort ? (m * 4 + 255) & ~(int64_t)255 : 0;
-    s->part_b = part_floats * 4;
-    return s->sort_b + s->coords_b + s->perm_b + s->part_b;
+    return s->sort_b + s->coords_b + s->perm_b;
 }
 
-static int evaluate_with(sg_grid *g, sg_eval_plan *p, const eval_scratch *s, char *base, int profile,
+static void whole_sums(sg_eval_plan *p)
+{
+    p->nshare = 1;
+    p->emit = SG_EMIT_SUM;
+    p->part_out = NULL;
+}
+
+/* The evaluation launches; base: the ordering's scratch, where it has any. */
+static int evaluate_with(sg_grid *g, sg_eval_plan *p, const sort_scratch *s, char *base, int profile,
                          const float *coords, float *out, int64_t m, cudaStream_t st)
 {
     const int32_t *perm = NULL;
@@ -888,7 +979,6 @@ static int evaluate_with(sg_grid *g, sg_eval_plan *p, const eval_scratch *s, cha
         coords = sorted;
     }
     if (profile) mark(g, SG_PHASE_EVALUATE, 0, st);
-    p->part_out = s->part_b ? (float *)(base + s->sort_b + s->coords_b + s->perm_b) : NULL;
     e = sgk_evaluate(p, coords, perm, out, m, st);
     if (e == cudaSuccess && p->nshare > 1) e = sgk_combine_one(p, perm, out, m, st);
     if (profile) mark(g, SG_PHASE_EVALUATE, 1, st);
@@ -898,22 +988,20 @@ static int evaluate_with(sg_grid *g, sg_eval_plan *p, const eval_scratch *s, cha
 static int evaluate_on(sg_grid *g, const float *coords, float *out, int64_t m, cudaStream_t st)
 {
     sg_eval_plan p;
-    eval_scratch s;
-    int64_t need, parts;
-    const int sort = plan_sort(g, m);
+    sort_scratch s;
+    int64_t need, sums;
     int r;
+    cudaError_t e;
     grid_plan(g, &p);
-    parts = plan_shares(g, m, &p);
-    need = scratch_plan(m, p.d, sort, parts, &s);
+    sums = plan_shares(g, m, &p);
+    need = scratch_plan(m, p.d, plan_sort(g, m), &s);
     r = need ? ensure(g, &g->d_scratch, &g->scratch_bytes, need, "evaluate scratch") : SG_OK;
-    if (r == SG_ERR_NOMEM && parts) {
-        /* no room for the segment sums: whole sums need none */
-        p.nshare = 1;
-        p.emit = SG_EMIT_SUM;
-        need = scratch_plan(m, p.d, sort, 0, &s);
-        r = need ? ensure(g, &g->d_scratch, &g->scratch_bytes, need, "evaluate scratch") : SG_OK;
-    }
-    return r == SG_OK ? evaluate_with(g, &p, &s, (char *)g->d_scratch, 1, coords, out, m, st) : r;
+    if (r != SG_OK) return r;
+    if (sums && !(p.part_out = sums_alloc(g, sums, st))) whole_sums(&p);
+    r = evaluate_with(g, &p, &s, (char *)g->d_scratch, 1, coords, out, m, st);
+    if (p.part_out && (e = cudaFreeAsync(p.part_out, st)) != cudaSuccess && r == SG_OK)
+        r = cuda_fail(e, "evaluate: returning the segment sums");
+    return r;
 }
 
 SG_API int sg_evaluate_device(sg_grid *g, const float *coords, float *out, int64_t m, void *stream)
@@ -935,10 +1023,10 @@ SG_API int sg_evaluate_device(sg_grid *g, const float *coords, float *out, int64
 SG_API int sg_evaluate_device_noalloc(sg_grid *g, const float *coords, float *out, int64_t m, void *stream)
 {
     sg_eval_plan p;
-    eval_scratch s;
-    int prev, r = SG_OK, e, sort;
+    sort_scratch s;
+    int prev, r = SG_OK, e;
     void *scratch = NULL;
-    int64_t have = 0, need, parts;
+    int64_t have = 0, need, sums;
     if (!g || m < 0 || (m > 0 && (!coords || !out))) return fail(SG_ERR_ARG, "sg_evaluate_device_noalloc: bad argument");
     if (!g->has_values || g->dev < 0)
         return fail(SG_ERR_STATE, "sg_evaluate_device_noalloc: the grid has no device state yet (set values first)");
@@ -948,18 +1036,13 @@ SG_API int sg_evaluate_device_noalloc(sg_grid *g, const float *coords, float *ou
     if (m == 0) return SG_OK;
     if ((r = enter(g, &prev)) != SG_OK) return r;
     grid_plan(g, &p);
-    parts = plan_shares(g, m, &p);
-    sort = plan_sort(g, m);
-    need = scratch_plan(m, g->L.d, sort, parts, &s);
+    sums = plan_shares(g, m, &p);
+    need = scratch_plan(m, g->L.d, plan_sort(g, m), &s);
     if ((e = sgk_noalloc_scratch(&scratch, &have)) != cudaSuccess) {
         r = cuda_fail((cudaError_t)e, "sg_evaluate_device_noalloc: scratch address");
     } else {
-        if (need > have && parts) {
-            /* the segment sums do not fit: whole sums */
-            p.nshare = 1;
-            p.emit = SG_EMIT_SUM;
-            need = scratch_plan(m, g->L.d, sort, 0, &s);
-        }
+        if (sums && need + sums * 4 <= have) p.part_out = (float *)((char *)scratch + need);
+        else whole_sums(&p);
         if (need > have)
             r = fail(SG_ERR_RANGE, "sg_evaluate_device_noalloc: %lld points in %d dims need more than the %lld-byte scratch",
                      (long long)m, g->L.d, (long long)have);

@@ -126,6 +126,10 @@ int sg_evaluate(sg_grid *grid, const float *coord_mat, float *out, int64_t num_e
 int sg_set_values_device(sg_grid *grid, const float *values, void *stream);
 int sg_get_values_device(sg_grid *grid, float *values, void *stream);
 int sg_hierarchize_async(sg_grid *grid, void *stream);
+/* Evaluations of one handle may overlap on several streams (once its values
+ * are in place: synchronize after the first evaluation of new values) with
+ * SG_OPT_EVAL_SORT 0 or one point per call; points that are ordered use
+ * scratch of the handle, and such calls have to be serialised. */
 int sg_evaluate_device(sg_grid *grid, const float *coord_mat, float *out,
                        int64_t num_evals, void *stream);
 /* Evaluation that allocates no memory, for callers that cannot call

@@ -1,0 +1,95 @@
+"""Evaluations of one grid that overlap on several streams, and evaluations
+recorded into CUDA graphs: whichever way a point's sum is added up, each call
+gives the bits that it gives alone."""
+import numpy as np
+import pytest
+
+import adaptive_sparse_grid_bench_b200 as sg
+from adaptive_sparse_grid_bench_b200 import inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(d, n):
+    g = sg.Grid(d, n)
+    g.set_values(inputs.uniform01(d * n, g.num_points) * 2 - 1)
+    g.hierarchize()
+    return g
+
+
+def _points(cuda, seed, m, d):
+    import torch
+    return torch.from_numpy(inputs.uniform_points(seed, m, d)).to(cuda)
+
+
+def _bits(t):
+    import torch
+    return t.view(torch.int32)
+
+
+# shared by segments and by parts; one point (never ordered) at the default options
+@pytest.mark.parametrize("d,n,m,sort", [(10, 8, 1000, 0), (10, 8, 60_000, 0), (6, 12, 700, 0), (10, 8, 1, 1)])
+def test_two_streams_on_one_grid(cuda, d, n, m, sort):
+    import torch
+    g = _grid(d, n)
+    g.set_option(sg.SG_OPT_EVAL_SORT, sort)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    X = [_points(cuda, 10 + i, m, d) for i in range(len(streams))]
+    alone = [torch.empty(m, device=cuda) for _ in streams]
+    for x, o in zip(X, alone):
+        g.evaluate_device(x, o)
+    g.sync()
+    torch.cuda.synchronize()
+    outs = [[torch.full((m,), np.nan, device=cuda) for _ in streams] for _ in range(8)]
+    torch.cuda.synchronize()
+    for row in outs:
+        for x, o, st in zip(X, row, streams):
+            g.evaluate_device(x, o, stream=st)
+    torch.cuda.synchronize()
+    for row in outs:
+        for o, a in zip(row, alone):
+            assert torch.equal(_bits(o), _bits(a))
+
+
+def test_smaller_call_after_a_larger_one_under_capture(cuda):
+    """What a call needs never grows as its points get fewer: after a call with
+    many points, one with fewer records into a graph, and the graph gives the
+    same bits after further calls of other sizes."""
+    import torch
+    d, n = 10, 8
+    g = _grid(d, n)
+    X = _points(cuda, 3, 100_000, d)
+    want = torch.empty(100_000, device=cuda)
+    g.evaluate_device(X, want)
+    g.sync()
+    out = torch.empty(50_000, device=cuda)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        g.evaluate_device(X, out, 50_000, torch.cuda.current_stream())
+    other = torch.empty(100_000, device=cuda)
+    for m in (1000, 20_000, 70_000):
+        g.evaluate_device(X, other, m)
+    g.sync()
+    for _ in range(2):
+        out.fill_(np.nan)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(_bits(out), _bits(want[:50_000]))
+
+
+def test_memory_of_shared_sums_is_given_back(cuda):
+    import torch
+
+    def cycle():
+        g = _grid(10, 8)
+        x, o = _points(cuda, 5, 50_000, 10), torch.empty(50_000, device=cuda)
+        g.evaluate_device(x, o)
+        g.sync()
+        used = torch.cuda.mem_get_info()[0]
+        g.close()
+        torch.cuda.synchronize()
+        return used, torch.cuda.mem_get_info()[0]
+
+    cycle()  # the allocator's own caches
+    first, second = cycle(), cycle()
+    assert first[1] == second[1] and first[1] > first[0]
