@@ -31,6 +31,14 @@ typedef struct sg_pass_state {
     uint16_t *combo_of;
 } sg_pass_state;
 
+/* The segment sums of a captured evaluation: its graph may be replayed beside
+ * any other call until the handle is destroyed, so each captured call has its
+ * own. */
+struct sg_captured_sums {
+    struct sg_captured_sums *next;
+    void *sums;
+};
+
 struct sg_grid {
     sg_layout L;
     int dev;        /* device of the device state, -1 before it exists */
@@ -58,6 +66,8 @@ struct sg_grid {
     cudaEvent_t ev[SG_NUM_PHASES][2]; /* profiling: start/stop per phase */
     int ev_used[SG_NUM_PHASES];
     cudaMemPool_t sums_pool; /* the device's pool of segment sums, once used  */
+    struct sg_captured_sums *captured;
+    int64_t captured_floats;
     uint32_t *d_sums;    /* segment table of the sums (sg_layout.h), NULL: one segment */
     sg_dev_alloc_fn alloc; /* NULL: cudaMalloc/cudaFree */
     sg_dev_free_fn free_fn;

@@ -138,30 +138,6 @@ static void pool_leave(int dev)
     pthread_mutex_unlock(&g_pool_mu);
 }
 
-/* Room for one evaluation's segment sums on st, NULL where there is none (whole
- * sums need none): out of memory, or st is capturing, where the memory would
- * have to outlive the call. */
-static float *sums_alloc(sg_grid *g, int64_t floats, cudaStream_t st)
-{
-    enum cudaStreamCaptureStatus cs;
-    enum cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    void *p = NULL;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return NULL;
-    }
-    /* another stream of the process may be capturing: allocating here does not
-     * concern it */
-    (void)cudaThreadExchangeStreamCaptureMode(&mode);
-    if (!g->sums_pool) g->sums_pool = pool_join(g->dev);
-    if (g->sums_pool && cudaMallocFromPoolAsync(&p, (size_t)floats * 4, g->sums_pool, st) != cudaSuccess) {
-        cudaGetLastError();
-        p = NULL;
-    }
-    (void)cudaThreadExchangeStreamCaptureMode(&mode);
-    return (float *)p;
-}
-
 static void free_device(sg_grid *g)
 {
     int k;
@@ -196,6 +172,12 @@ static void free_device(sg_grid *g)
     dev_free(g, g->d_sums);
     if (g->sums_pool) pool_leave(g->dev);
     g->sums_pool = NULL;
+    while (g->captured) {
+        struct sg_captured_sums *c = g->captured;
+        g->captured = c->next;
+        dev_free(g, c->sums);
+        free(c);
+    }
 }
 
 int sg_create_with_allocator(int d, int n, const int *limits, sg_dev_alloc_fn alloc, sg_dev_free_fn free_fn,
@@ -342,6 +324,53 @@ static int enter(sg_grid *g, int *prev)
 static void leave(sg_grid *g, int prev)
 {
     if (g->dev >= 0 && g->dev != prev) cudaSetDevice(prev);
+}
+
+/* A captured evaluation's segment sums: as much for all of a handle's captured
+ * calls as for one largest call. */
+static void *captured_sums_alloc(sg_grid *g, int64_t floats)
+{
+    struct sg_captured_sums *c;
+    if (g->captured_floats + floats > SG_SHARE_FLOATS) return NULL;
+    c = (struct sg_captured_sums *)malloc(sizeof(*c));
+    if (!c) return NULL;
+    if (dev_alloc(g, &c->sums, floats * 4, "segment sums of a captured evaluation") != SG_OK) {
+        free(c);
+        return NULL;
+    }
+    g->captured_floats += floats;
+    c->next = g->captured;
+    g->captured = c;
+    return c->sums;
+}
+
+/* Room for one evaluation's segment sums on st, NULL where there is none (whole
+ * sums need none).  *ours: to be returned to the pool after the evaluation. */
+static float *sums_alloc(sg_grid *g, int64_t floats, cudaStream_t st, int *ours)
+{
+    enum cudaStreamCaptureStatus cs;
+    enum cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    void *p = NULL;
+    *ours = 0;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs == cudaStreamCaptureStatusInvalidated) {
+        cudaGetLastError();
+        return NULL;
+    }
+    /* st, or another stream of the process, may be capturing: allocating here
+     * does not concern it */
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cs == cudaStreamCaptureStatusActive) {
+        p = captured_sums_alloc(g, floats);
+    } else {
+        if (!g->sums_pool) g->sums_pool = pool_join(g->dev);
+        if (g->sums_pool && cudaMallocFromPoolAsync(&p, (size_t)floats * 4, g->sums_pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            p = NULL;
+        }
+        *ours = p != NULL;
+    }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return (float *)p;
 }
 
 static int dev_upload(sg_grid *g, void **p, const void *src, int64_t bytes, cudaStream_t st, const char *what)
@@ -990,16 +1019,16 @@ static int evaluate_on(sg_grid *g, const float *coords, float *out, int64_t m, c
     sg_eval_plan p;
     sort_scratch s;
     int64_t need, sums;
-    int r;
+    int r, ours = 0;
     cudaError_t e;
     grid_plan(g, &p);
     sums = plan_shares(g, m, &p);
     need = scratch_plan(m, p.d, plan_sort(g, m), &s);
     r = need ? ensure(g, &g->d_scratch, &g->scratch_bytes, need, "evaluate scratch") : SG_OK;
     if (r != SG_OK) return r;
-    if (sums && !(p.part_out = sums_alloc(g, sums, st))) whole_sums(&p);
+    if (sums && !(p.part_out = sums_alloc(g, sums, st, &ours))) whole_sums(&p);
     r = evaluate_with(g, &p, &s, (char *)g->d_scratch, 1, coords, out, m, st);
-    if (p.part_out && (e = cudaFreeAsync(p.part_out, st)) != cudaSuccess && r == SG_OK)
+    if (ours && (e = cudaFreeAsync(p.part_out, st)) != cudaSuccess && r == SG_OK)
         r = cuda_fail(e, "evaluate: returning the segment sums");
     return r;
 }

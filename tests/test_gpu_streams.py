@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import adaptive_sparse_grid_bench_b200 as sg
-from adaptive_sparse_grid_bench_b200 import inputs
+from adaptive_sparse_grid_bench_b200 import _lib, inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -75,6 +75,53 @@ def test_smaller_call_after_a_larger_one_under_capture(cuda):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(_bits(out), _bits(want[:50_000]))
+
+
+def test_captured_evaluations_share_their_sums(cuda):
+    """A captured call keeps its sums in memory of its own: two graphs of one grid
+    and an eager call run side by side.  Where the handle has no more room for
+    such memory the call takes whole sums: one launch less, the same bits."""
+    import torch
+    d, n, m = 10, 8, 60_000
+    g = _grid(d, n)
+    g.set_option(sg.SG_OPT_EVAL_SORT, 0)
+    X = [_points(cuda, 20 + i, m, d) for i in range(3)]
+    want = [torch.empty(m, device=cuda) for _ in X]
+    for x, o in zip(X, want):
+        g.evaluate_device(x, o)
+    g.sync()
+    got = [torch.empty(m, device=cuda) for _ in X]
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+    for k, graph in enumerate(graphs):
+        with torch.cuda.graph(graph):
+            before = _lib.kernel_launches()
+            g.evaluate_device(X[k], got[k], m, torch.cuda.current_stream())
+            assert _lib.kernel_launches() - before == 2  # the sums, and adding them up
+    streams = [torch.cuda.Stream() for _ in X]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for k, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                if k < len(graphs):
+                    graphs[k].replay()
+                else:
+                    g.evaluate_device(X[k], got[k], m, st)
+    torch.cuda.synchronize()
+    for o, w in zip(got, want):
+        assert torch.equal(_bits(o), _bits(w))
+    # 128 segments x 10,000 points x 4 bytes: room for 24 more beside these two
+    launches = []
+    for _ in range(30):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            before = _lib.kernel_launches()
+            g.evaluate_device(X[0], got[0], 10_000, torch.cuda.current_stream())
+            launches.append(_lib.kernel_launches() - before)
+        got[0].fill_(np.nan)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(_bits(got[0][:10_000]), _bits(want[0][:10_000]))
+    assert launches[0] == 2 and launches[-1] == 1
 
 
 def test_memory_of_shared_sums_is_given_back(cuda):
