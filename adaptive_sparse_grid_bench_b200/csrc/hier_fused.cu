@@ -209,7 +209,10 @@ template <typename T, int G, int NT>
 int launch_nt(T *a, const sg_unit_pass *p, cudaStream_t st)
 {
     const int64_t smem = p->max_elems * (int64_t)sizeof(T);
-    cudaError_t e = cudaFuncSetAttribute(k_sweep_fused<T, G, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    /* the limit is one for the process, so always the same value: set to this
+     * launch's size it could be lowered by another thread before the launch */
+    cudaError_t e = cudaFuncSetAttribute(k_sweep_fused<T, G, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SG_UNIT_MAX_BYTES);
     if (e != cudaSuccess) return e;
     k_sweep_fused<T, G, NT><<<(unsigned)p->nunits, NT, (size_t)smem, st>>>(a, p->units, p->offs, p->tables);
     sgk_count(1);

@@ -124,7 +124,9 @@ template <typename T, int NT>
 int launch_nt(float *a, const sg_smem_grid *grids, int ngrids, const sg_chain *chains, const uint32_t *seg, size_t smem,
               void *stream)
 {
-    cudaError_t e = cudaFuncSetAttribute(k_hier_smem<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    /* not `smem`: the limit is one for all threads of the process */
+    cudaError_t e = cudaFuncSetAttribute(k_hier_smem<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SG_SMEM_GRID_MAX_BYTES);
     if (e != cudaSuccess) return e;
     k_hier_smem<T, NT><<<ngrids, NT, smem, (cudaStream_t)stream>>>(a, grids, chains, seg);
     sgk_count(1);

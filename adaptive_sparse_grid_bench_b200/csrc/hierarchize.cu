@@ -432,6 +432,11 @@ __global__ void __launch_bounds__(256) k_copy_groups(const float *__restrict__ s
 int g_num_sms = 0;
 long long g_launches = 0;
 
+/* Largest dynamic shared memory of a launch.  The kernels' limits are set to
+ * it, not to a launch's own size: a limit is one for the process, and another
+ * thread's launch would lower it between this one's setting and its launch. */
+constexpr int kMaxSmem = 200 * 1024;
+
 template <typename T, int NT>
 int launch_chains_nt(T *a, const sg_sweep_tables *t, int64_t cap, int *err, long long wait_limit, int stall,
                      void *stream)
@@ -442,8 +447,8 @@ int launch_chains_nt(T *a, const sg_sweep_tables *t, int64_t cap, int *err, long
     nst = nst < 2 ? 2 : (nst > kMaxStages ? kMaxStages : nst);
     const int64_t smem = nst * stage_bytes;
     const int capi = (int)(stage_bytes / (int64_t)sizeof(T));
-    cudaError_t e = cudaFuncSetAttribute(k_sweep_chains<T, NT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_sweep_chains<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kMaxSmem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chains<T, NT>, NT, (size_t)smem);
@@ -548,8 +553,8 @@ int launch_small(T *a, const sg_sweep_tables *t, void *stream)
     if (t->nchains == 0) return cudaSuccess;
     const int64_t cap = sizeof(T) == 4 ? t->cap32 : t->cap64;
     const int64_t smem = 8 * cap * (int64_t)sizeof(T); /* 8 warps per CTA */
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_sweep_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(k_sweep_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_small<T>, 256, (size_t)smem);
@@ -601,7 +606,7 @@ int64_t sgk_chain_smem_bytes(int64_t cap_elems, int elem_bytes)
 {
     const int64_t stage = (cap_elems * elem_bytes + 127) / 128 * 128;
     const int64_t total = 2 * stage;
-    return total <= 200 * 1024 ? total : -1;
+    return total <= kMaxSmem ? total : -1;
 }
 
 int sgk_sweep_chains_f32(float *a, const sg_sweep_tables *t, int *err, void *stream)
@@ -628,7 +633,7 @@ int sgk_sweep_small_f64(double *a, const sg_sweep_tables *t, void *stream)
 int64_t sgk_small_smem_bytes(int64_t cap_elems, int elem_bytes)
 {
     const int64_t b = 8 * cap_elems * elem_bytes;
-    return b <= 200 * 1024 ? b : -1;
+    return b <= kMaxSmem ? b : -1;
 }
 int sgk_sweep_gather_f32(float *a, const sg_sweep_tables *t, void *stream)
 {
