@@ -560,20 +560,54 @@ bad:
     return r;
 }
 
+/* Whether a kernel on the handle's device may touch the floats [p, p + count):
+ * this device's own or managed memory, all inside one allocation, float-aligned.
+ * A copy checks or handles the rest (another GPU's memory without peer access,
+ * host memory, short buffers, odd addresses); a kernel would fault on it. */
+typedef int (*range_fn)(unsigned long long *base, size_t *size, unsigned long long p); /* cuMemGetAddressRange */
+static range_fn g_range;
+static pthread_once_t g_range_once = PTHREAD_ONCE_INIT;
+
+static void find_range_fn(void)
+{
+    void *f = NULL;
+    enum cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+        g_range = (range_fn)f;
+    else
+        cudaGetLastError();
+}
+
+static int kernel_may_touch(const sg_grid *g, const void *p, int64_t count)
+{
+    struct cudaPointerAttributes a;
+    unsigned long long base = 0, at = (unsigned long long)(uintptr_t)p;
+    size_t size = 0;
+    if (at % sizeof(float)) return 0;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (a.type != cudaMemoryTypeManaged && !(a.type == cudaMemoryTypeDevice && a.device == g->dev)) return 0;
+    pthread_once(&g_range_once, find_range_fn);
+    return g_range && g_range(&base, &size, at) == 0 && at + (unsigned long long)count * 4 <= base + size;
+}
+
 /* Copies the N compact values into (or out of) the group-aligned layout: one
  * contiguous copy per level group.  Between device buffers one kernel moves the
  * groups below 2^24 values: n copies of two microseconds each were more than
  * half the time of a small grid's hierarchization (d = 4, n = 8: 25 us each way,
  * 4 us in one kernel; d = 10, n = 10: 85 and 65 us).  The copy engine path is
  * the faster one for larger groups (d = 6, n = 14, limits 9: 185 us, 201 us by
- * the kernel). */
+ * the kernel), and the one for buffers that the kernel must not touch. */
 #define SG_GROUP_COPY ((int64_t)1 << 24)
 static int copy_groups(sg_grid *g, float *dst, const float *src, int to_device, enum cudaMemcpyKind kind,
                        cudaStream_t st)
 {
     const sg_layout *L = &g->L;
     int s, small = 0, e;
-    if (kind == cudaMemcpyDeviceToDevice) {
+    if (kind == cudaMemcpyDeviceToDevice && kernel_may_touch(g, to_device ? src : dst, L->N)) {
         while (small < L->n && L->lidx[small + 1] - L->lidx[small] < SG_GROUP_COPY) small++;
         if ((e = sgk_copy_groups(L, small, src, dst, !to_device, st)) != cudaSuccess)
             return cuda_fail((cudaError_t)e, "grid values");
