@@ -29,6 +29,7 @@ typedef struct sg_pass_state {
     sg_unit_combo *combos;
     sg_unit_node *nodes;
     uint16_t *combo_of;
+    int64_t bytes; /* of the five */
 } sg_pass_state;
 
 /* The segment sums of a captured evaluation: its graph may be replayed beside

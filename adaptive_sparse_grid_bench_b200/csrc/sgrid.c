@@ -138,6 +138,17 @@ static void pool_leave(int dev)
     pthread_mutex_unlock(&g_pool_mu);
 }
 
+static void pass_free(sg_grid *g, sg_pass_state *ps)
+{
+    dev_free(g, ps->units);
+    dev_free(g, ps->offs);
+    dev_free(g, ps->combos);
+    dev_free(g, ps->nodes);
+    dev_free(g, ps->combo_of);
+    g->dev_bytes -= ps->bytes;
+    memset(ps, 0, sizeof(*ps));
+}
+
 static void free_device(sg_grid *g)
 {
     int k;
@@ -158,13 +169,7 @@ static void free_device(sg_grid *g)
         int f;
         dev_free(g, g->d_chains[k]);
         dev_free(g, g->d_seg[k]);
-        for (f = 0; f < 2; f++) {
-            dev_free(g, g->pass[f][k].units);
-            dev_free(g, g->pass[f][k].offs);
-            dev_free(g, g->pass[f][k].combos);
-            dev_free(g, g->pass[f][k].nodes);
-            dev_free(g, g->pass[f][k].combo_of);
-        }
+        for (f = 0; f < 2; f++) pass_free(g, &g->pass[f][k]);
     }
     dev_free(g, g->d_err);
     dev_free(g, g->d_scratch);
@@ -373,6 +378,15 @@ static float *sums_alloc(sg_grid *g, int64_t floats, cudaStream_t st, int *ours)
     return (float *)p;
 }
 
+/* Undoes a dev_alloc of `bytes` (nothing where *p is NULL). */
+static void dev_drop(sg_grid *g, void **p, int64_t bytes)
+{
+    if (!*p) return;
+    dev_free(g, *p);
+    g->dev_bytes -= bytes;
+    *p = NULL;
+}
+
 static int dev_upload(sg_grid *g, void **p, const void *src, int64_t bytes, cudaStream_t st, const char *what)
 {
     cudaError_t e;
@@ -380,7 +394,9 @@ static int dev_upload(sg_grid *g, void **p, const void *src, int64_t bytes, cuda
     if (r != SG_OK || bytes <= 0) return r;
     /* pageable source: the copy has taken the bytes when the call returns */
     e = cudaMemcpyAsync(*p, src, (size_t)bytes, cudaMemcpyHostToDevice, st);
-    return e == cudaSuccess ? SG_OK : cuda_fail(e, what);
+    if (e == cudaSuccess) return SG_OK;
+    dev_drop(g, p, bytes);
+    return cuda_fail(e, what);
 }
 
 /* The chain table of dim k (single-dim sweeps). */
@@ -411,7 +427,10 @@ static int build_chains(sg_grid *g, int k, cudaStream_t st)
         r = dev_upload(g, (void **)&g->d_chains[k], ch, nch * (int64_t)sizeof(sg_chain), st, "sweep chains");
     free(ch);
     free(seg);
-    if (r != SG_OK) return r;
+    if (r != SG_OK) {
+        dev_drop(g, (void **)&g->d_seg[k], nseg * 4); /* the next attempt starts afresh */
+        return r;
+    }
     g->sweep[k].chains = g->d_chains[k];
     g->sweep[k].seg = g->d_seg[k];
     g->sweep[k].nchains = nch;
@@ -421,21 +440,23 @@ static int build_chains(sg_grid *g, int k, cudaStream_t st)
     return SG_OK;
 }
 
-/* The passes of the current precision (f: 0 FP32, 1 FP64). */
+/* The passes of the current precision (f: 0 FP32, 1 FP64): all of them or, on
+ * failure, none. */
 static int build_passes(sg_grid *g, int f, cudaStream_t st)
 {
     const sg_layout *L = &g->L;
-    int k, r, n = 0;
+    int k, r = SG_OK, n = 0;
     if (g->npass[f]) return SG_OK;
-    for (k = 0; k < L->d; n++) {
+    for (k = 0; k < L->d && r == SG_OK; n++) {
         sg_pass_state *ps = &g->pass[f][n];
+        const int64_t before = g->dev_bytes;
         sg_pass_host h;
         const int dims = sg_layout_pass_dims(L, k, f ? 8 : 4);
         ps->k0 = k;
         ps->p.g = dims;
         k += dims ? dims : 1;
         if (!dims) {
-            if ((r = build_chains(g, ps->k0, st)) != SG_OK) return r;
+            r = build_chains(g, ps->k0, st);
             continue;
         }
         r = sg_layout_pass(L, ps->k0, dims, &h);
@@ -454,10 +475,15 @@ static int build_passes(sg_grid *g, int f, cudaStream_t st)
         ps->p.tables.nodes = ps->nodes;
         ps->p.tables.combo_of = ps->combo_of;
         sg_layout_pass_free(&h);
-        if (r != SG_OK) return r;
+        ps->bytes = g->dev_bytes - before;
     }
-    g->npass[f] = n;
-    return SG_OK;
+    if (r == SG_OK) {
+        g->npass[f] = n;
+    } else {
+        cudaStreamSynchronize(st); /* the uploads of what is freed */
+        while (n-- > 0) pass_free(g, &g->pass[f][n]);
+    }
+    return r;
 }
 
 /* The sweep tables that the handle's options call for. */

@@ -1,0 +1,126 @@
+"""The library's host code over a CUDA runtime in host memory (fake_cuda.c): what
+it allocates when an allocation fails, which streams its calls touch, and how
+often it allocates.  No GPU."""
+import ctypes as C
+import os
+import re
+import subprocess
+
+import numpy as np
+import pytest
+
+from adaptive_sparse_grid_bench_b200 import _lib
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "adaptive_sparse_grid_bench_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    out = tmp_path_factory.mktemp("fake")
+    cc = ["gcc", "-O1", "-fPIC", "-std=gnu11", "-I", os.path.join(CUDA, "include"), "-I", CSRC]
+    objs = []
+    for src in [os.path.join(CSRC, f) for f in ("sgrid.c", "sgrid_batch.c", "sg_layout.c")] + [
+            os.path.join(ROOT, "tests", "fake_cuda.c")]:
+        objs.append(str(out / (os.path.basename(src)[:-2] + ".o")))
+        subprocess.run(cc + ["-c", src, "-o", objs[-1]], check=True)
+    names = subprocess.run(["nm"] + objs, check=True, capture_output=True, text=True).stdout
+    wanted = set(re.findall(r" U (sgk_\w+)", names)) - set(re.findall(r" T (sgk_\w+)", names))
+    empty = out / "empty.c"
+    empty.write_text("".join(f"int {n}() {{ return 0; }}\n" for n in sorted(wanted)))
+    lib = str(out / "libfake.so")
+    subprocess.run(cc + ["-shared", str(empty)] + objs + ["-o", lib, "-lpthread"], check=True)
+    so = C.CDLL(lib)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        if hasattr(so, name):
+            getattr(so, name).restype, getattr(so, name).argtypes = res, args
+    for name in ("live", "pool_live", "allocs", "frees", "legacy", "waits", "unsafe"):
+        getattr(so, "fake_" + name).restype = C.c_long
+    so.fake_fail.argtypes = [C.c_long]
+    so.fake_capture.argtypes = [C.c_void_p]
+    return so
+
+
+class Grid:
+    def __init__(self, so, d, n):
+        self.so, self.h, self.d = so, C.c_void_p(), d
+        assert so.sg_create(d, n, None, C.byref(self.h)) == _lib.SG_OK
+        v = C.c_int64()
+        so.sg_num_points(self.h, C.byref(v))
+        self.values = np.zeros(v.value, np.float32)
+
+    def set_values(self):
+        return self.so.sg_set_values(self.h, self.values.ctypes.data)
+
+    def hierarchize(self):
+        return self.so.sg_hierarchize(self.h)
+
+    def device_bytes(self):
+        v = C.c_int64()
+        self.so.sg_device_bytes(self.h, C.byref(v))
+        return v.value
+
+    def close(self):
+        self.so.sg_destroy(self.h)
+
+
+def _until_no_failure(fake, attempt):
+    """Calls attempt() with its first, second, ... allocation failing until none
+    does; yields after every failure."""
+    k = 0
+    while True:
+        fake.fake_fail(k)
+        r = attempt()
+        fake.fake_fail(-1)
+        if r == _lib.SG_OK:
+            return
+        assert r == _lib.SG_ERR_NOMEM, k
+        k += 1
+        yield k
+
+
+SHAPES = [(6, 6), (3, 8), (5, 11)]  # passes of several dims; single-dim sweeps; both
+
+
+@pytest.mark.parametrize("d,n", SHAPES)
+def test_failed_set_up_leaves_nothing_allocated(fake, d, n):
+    start = fake.fake_live()
+    g = Grid(fake, d, n)
+    fails = 0
+    for fails in _until_no_failure(fake, g.set_values):
+        assert fake.fake_live() == start and g.device_bytes() == 0
+    assert fails > 5
+    g.close()
+    assert fake.fake_live() == start
+
+
+@pytest.mark.parametrize("d,n", SHAPES)
+@pytest.mark.parametrize("option,value", [(_lib.SG_OPT_HIER_PRECISION, _lib.SG_HIER_FP64),
+                                          (_lib.SG_OPT_HIER_KERNEL, 2)])
+def test_failed_tables_are_not_lost(fake, d, n, option, value):
+    """Tables of another option, built on a live grid: an attempt that fails
+    halfway and is made again leaves nothing behind that is not freed with the
+    grid."""
+    start, k = fake.fake_live(), 0
+    while True:
+        g = Grid(fake, d, n)
+        assert g.set_values() == _lib.SG_OK
+        fake.fake_fail(k)
+        r = fake.sg_set_option(g.h, option, value)
+        if r == _lib.SG_OK:
+            r = g.hierarchize()
+        fake.fake_fail(-1)
+        assert r in (_lib.SG_OK, _lib.SG_ERR_NOMEM)
+        assert fake.sg_set_option(g.h, option, value) == _lib.SG_OK and g.hierarchize() == _lib.SG_OK
+        held = g.device_bytes()
+        g.close()
+        assert fake.fake_live() == start, k
+        if r == _lib.SG_OK:
+            break
+        if k == 0:
+            first = held
+        assert held == first
+        k += 1
+    if (d, option) != (3, _lib.SG_OPT_HIER_KERNEL):  # (3, 8) has its chains already
+        assert k > 0
