@@ -486,14 +486,27 @@ static int build_passes(sg_grid *g, int f, cudaStream_t st)
     return r;
 }
 
+/* The options call for single-dim sweeps throughout. */
+static int single_sweeps(const sg_grid *g)
+{
+    return g->opt[SG_OPT_HIER_KERNEL] == 2 || g->opt[SG_OPT_TEST_WAIT] > 0;
+}
+
 /* The sweep tables that the handle's options call for. */
+static int sweeps_built(const sg_grid *g)
+{
+    int k;
+    if (!single_sweeps(g)) return g->npass[g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64] > 0;
+    for (k = 0; k < g->L.d; k++)
+        if (!g->d_chains[k]) return 0;
+    return 1;
+}
+
 static int build_sweeps(sg_grid *g, cudaStream_t st)
 {
     int k, r = SG_OK;
-    if (g->opt[SG_OPT_HIER_KERNEL] == 2 || g->opt[SG_OPT_TEST_WAIT] > 0)
-        for (k = 0; k < g->L.d && r == SG_OK; k++) r = build_chains(g, k, st);
-    else
-        r = build_passes(g, g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64, st);
+    if (!single_sweeps(g)) return build_passes(g, g->opt[SG_OPT_HIER_PRECISION] == SG_HIER_FP64, st);
+    for (k = 0; k < g->L.d && r == SG_OK; k++) r = build_chains(g, k, st);
     return r;
 }
 
@@ -856,10 +869,12 @@ SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_
     tune_eval_arg ta;
     double t[SG_TUNE_TIMINGS], best = 1e30;
     float *saved = NULL;
+    int64_t opt[NOPT];
     int prev, r = SG_OK, i, j, k, chains_apply = 0, bi = -1;
     if (!g || !coords || !out || num_evals < 1) return fail(SG_ERR_ARG, "sg_autotune: bad argument");
     if (!g->has_values) return fail(SG_ERR_STATE, "sg_autotune: no values have been set");
     if ((r = enter(g, &prev)) != SG_OK) return r;
+    memcpy(opt, g->opt, sizeof(opt));
     for (i = 0; i < SG_TUNE_TIMINGS; i++) t[i] = -1.0;
     ta.coords = coords;
     ta.out = out;
@@ -916,6 +931,7 @@ SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_
     }
     if (saved) dev_free(g, saved);
     if (saved) g->dev_bytes -= g->L.Npad * 4;
+    if (r != SG_OK) memcpy(g->opt, opt, sizeof(opt)); /* settings whose tables exist */
     if (ms)
         for (i = 0; i < SG_TUNE_TIMINGS; i++) ms[i] = t[i];
     leave(g, prev);
@@ -1233,6 +1249,37 @@ SG_API int sg_gp2idx_device(const sg_grid *g, const int *levels, const int *indi
     return SG_OK;
 }
 
+/* Sets an option that chooses the sweep tables and builds those a live handle
+ * lacks, here rather than in a hierarchization that may be under stream
+ * capture: on a stream of their own, so that neither the legacy stream's work
+ * nor a capture is waited for or disturbed.  On failure the option keeps its
+ * value, whose tables exist. */
+static int set_sweep_option(sg_grid *g, int option, int64_t value)
+{
+    const int64_t old = g->opt[option];
+    enum cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaStream_t st = NULL;
+    cudaError_t e;
+    int prev, r = SG_OK;
+    g->opt[option] = value;
+    if (g->dev < 0 || sweeps_built(g)) return SG_OK;
+    if ((r = enter(g, &prev)) == SG_OK) {
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) {
+            r = cuda_fail(e, "sg_set_option: stream");
+        } else {
+            r = build_sweeps(g, st);
+            e = cudaStreamSynchronize(st);
+            if (r == SG_OK && e != cudaSuccess) r = cuda_fail(e, "uploading sweep tables");
+            cudaStreamDestroy(st);
+        }
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        leave(g, prev);
+    }
+    if (r != SG_OK) g->opt[option] = old;
+    return r;
+}
+
 SG_API int sg_set_option(sg_grid *g, int option, int64_t value)
 {
     if (!g) return fail(SG_ERR_ARG, "sg_set_option: NULL grid");
@@ -1261,17 +1308,9 @@ SG_API int sg_set_option(sg_grid *g, int option, int64_t value)
     default:
         return fail(SG_ERR_ARG, "unknown option %d", option);
     }
+    if (option == SG_OPT_HIER_PRECISION || option == SG_OPT_HIER_KERNEL || option == SG_OPT_TEST_WAIT)
+        return set_sweep_option(g, option, value);
     g->opt[option] = value;
-    if (g->dev >= 0 && (option == SG_OPT_HIER_PRECISION || option == SG_OPT_HIER_KERNEL || option == SG_OPT_TEST_WAIT)) {
-        /* the sweep tables of the new setting, here rather than in a
-         * hierarchization that may be under stream capture */
-        int prev, r = enter(g, &prev);
-        if (r != SG_OK) return r;
-        r = build_sweeps(g, 0);
-        if (r == SG_OK && cudaStreamSynchronize(0) != cudaSuccess) r = cuda_fail(cudaGetLastError(), "uploading sweep tables");
-        leave(g, prev);
-        return r;
-    }
     return SG_OK;
 }
 

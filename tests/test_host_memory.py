@@ -124,3 +124,28 @@ def test_failed_tables_are_not_lost(fake, d, n, option, value):
         k += 1
     if (d, option) != (3, _lib.SG_OPT_HIER_KERNEL):  # (3, 8) has its chains already
         assert k > 0
+
+
+def test_options_change_whole_or_not_at_all(fake):
+    """A setting whose tables cannot be built is refused and the old one stays,
+    under which the grid still works.  The tables' uploads touch neither the
+    legacy stream nor a stream that is capturing."""
+    g = Grid(fake, 6, 6)
+    assert g.set_values() == _lib.SG_OK
+    v = C.c_int64()
+    for option, value in ((_lib.SG_OPT_HIER_PRECISION, _lib.SG_HIER_FP64), (_lib.SG_OPT_HIER_KERNEL, 2)):
+        fake.fake_fail(1)
+        assert fake.sg_set_option(g.h, option, value) == _lib.SG_ERR_NOMEM
+        assert fake.sg_get_option(g.h, option, C.byref(v)) == _lib.SG_OK and v.value == 0
+        allocs = fake.fake_allocs()
+        assert fake.sg_hierarchize_async(g.h, None) == _lib.SG_OK and fake.fake_allocs() == allocs
+    legacy, unsafe = fake.fake_legacy(), fake.fake_unsafe()
+    fake.fake_capture(12345)
+    try:
+        for option, value in ((_lib.SG_OPT_HIER_PRECISION, _lib.SG_HIER_FP64), (_lib.SG_OPT_HIER_KERNEL, 2),
+                              (_lib.SG_OPT_HIER_PRECISION, _lib.SG_HIER_FP32), (_lib.SG_OPT_HIER_KERNEL, 0)):
+            assert fake.sg_set_option(g.h, option, value) == _lib.SG_OK
+    finally:
+        fake.fake_capture(None)
+    assert (fake.fake_legacy(), fake.fake_unsafe()) == (legacy, unsafe)
+    g.close()
