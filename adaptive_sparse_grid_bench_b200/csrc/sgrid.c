@@ -1082,6 +1082,8 @@ static int evaluate_with(sg_grid *g, sg_eval_plan *p, const sort_scratch *s, cha
             return cuda_fail((cudaError_t)e, "sorting query points");
         if (profile) mark(g, SG_PHASE_SORT, 1, st);
         coords = sorted;
+    } else if (profile && g->opt[SG_OPT_PROFILE]) {
+        g->ev_used[SG_PHASE_SORT] = 0; /* not a phase of this call */
     }
     if (profile) mark(g, SG_PHASE_EVALUATE, 0, st);
     e = sgk_evaluate(p, coords, perm, out, m, st);

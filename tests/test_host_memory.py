@@ -149,3 +149,17 @@ def test_options_change_whole_or_not_at_all(fake):
         fake.fake_capture(None)
     assert (fake.fake_legacy(), fake.fake_unsafe()) == (legacy, unsafe)
     g.close()
+
+
+def test_timings_are_of_the_latest_call(fake):
+    """A call that does not order its points has no ordering time, whatever an
+    earlier one had."""
+    g = Grid(fake, 6, 9)
+    assert g.set_values() == _lib.SG_OK
+    assert fake.sg_set_option(g.h, _lib.SG_OPT_PROFILE, 1) == _lib.SG_OK
+    x, ms = np.zeros((60_000, 6), np.float32), np.zeros(_lib.SG_NUM_PHASES)
+    for m, ordered in ((60_000, True), (10, False), (60_000, True), (1, False)):
+        assert fake.sg_evaluate_device(g.h, x.ctypes.data, x.ctypes.data, m, None) == _lib.SG_OK
+        assert fake.sg_timings(g.h, ms.ctypes.data) == _lib.SG_OK
+        assert (ms[1] >= 0) == ordered and ms[2] >= 0, m
+    g.close()
