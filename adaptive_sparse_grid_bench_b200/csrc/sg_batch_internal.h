@@ -59,7 +59,7 @@ struct sg_batch {
     uint32_t *d_seg;                 /* segment tables (sg_layout.h)                */
     float *d_part;                   /* parts or segments of shared sums            */
     int64_t part_floats;
-    int32_t *d_citems;               /* combine CTAs of the shared sums             */
+    const int32_t *d_citems;         /* combine CTAs of the shared sums, in d_items */
     int ncitems;
     sg_eval_args *h_eval_args, *d_eval_args;
     int32_t *h_items, *d_items;

@@ -123,10 +123,8 @@ static void free_dev(sg_batch *b)
     cudaFree(b->d_rsrc);
     cudaFree(b->d_seg);
     cudaFree(b->d_part);
-    cudaFree(b->d_citems);
     b->d_seg = NULL;
     b->d_part = NULL;
-    b->d_citems = NULL;
     b->part_floats = 0;
     cudaFree(b->d_smem_grids);
     cudaFree(b->d_smem_chains);
@@ -944,7 +942,6 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
 {
     int g, k, r, q;
     int64_t coff = 0, ni = 0, cap_items = 0, ctas = 0, parts = 0, nc = 0, cap_c = 0;
-    int32_t *citems;
     int same = b->h_eval_args && b->eval_coords == coords && b->eval_out == out && b->eval_sort == b->sort;
     for (g = 0; same && g <= b->ng; g++) same = b->eval_pt_off[g] == pt_off[g];
     if (same) return SG_OK;
@@ -996,7 +993,7 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
         qsort_r(b->order, (size_t)b->ng, sizeof(int), cmp_dim_then_subspaces, b);
     }
     free(b->h_items);
-    b->h_items = (int32_t *)malloc((size_t)(cap_items > 0 ? cap_items : 1) * 2 * sizeof(int32_t));
+    b->h_items = (int32_t *)malloc((size_t)(cap_items + cap_c > 0 ? cap_items + cap_c : 1) * 2 * sizeof(int32_t));
     if (!b->h_items) return bfail(SG_ERR_NOMEM, "out of host memory");
     for (g = 0; g < b->ng; g++) {
         const sg_layout *L = &b->L[g];
@@ -1048,37 +1045,30 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
         }
         b->items_count[k] = (int)ni - b->items_first[k];
     }
-    if (ni > b->items_cap) {
+    /* behind them the combine CTAs of the grids with shared sums: a plan for
+     * other offsets or buffers allocates nothing that it has room for */
+    for (g = 0; g < b->ng; g++) {
+        int64_t p;
+        if (b->h_eval_args[g].nshare <= 1) continue;
+        for (p = 0; p < pt_off[g + 1] - pt_off[g]; p += 256) {
+            b->h_items[2 * (ni + nc)] = g;
+            b->h_items[2 * (ni + nc) + 1] = (int32_t)p;
+            nc++;
+        }
+    }
+    if (ni + nc > b->items_cap) {
         cudaFree(b->d_items);
         b->d_items = NULL;
-        if ((r = balloc(b, (void **)&b->d_items, ni * 2 * 4, "batch eval items")) != SG_OK) return r;
-        b->items_cap = ni;
+        b->dev_bytes -= b->items_cap * 8;
+        b->items_cap = 0;
+        if ((r = balloc(b, (void **)&b->d_items, (ni + nc) * 8, "batch eval items")) != SG_OK) return r;
+        b->items_cap = ni + nc;
     }
     BCU(cudaMemcpy(b->d_eval_args, b->h_eval_args, (size_t)b->ng * sizeof(sg_eval_args), cudaMemcpyHostToDevice),
         "upload eval args");
-    if (ni > 0) BCU(cudaMemcpy(b->d_items, b->h_items, (size_t)ni * 2 * 4, cudaMemcpyHostToDevice), "upload items");
-    /* combine CTAs of the grids with shared sums */
-    cudaFree(b->d_citems);
-    b->d_citems = NULL;
-    b->dev_bytes -= (int64_t)b->ncitems * 8;
-    b->ncitems = 0;
-    if (cap_c > 0) {
-        citems = (int32_t *)malloc((size_t)cap_c * 8);
-        if (!citems) return bfail(SG_ERR_NOMEM, "out of host memory");
-        for (g = 0; g < b->ng; g++) {
-            int64_t p;
-            if (b->h_eval_args[g].nshare <= 1) continue;
-            for (p = 0; p < pt_off[g + 1] - pt_off[g]; p += 256) {
-                citems[2 * nc] = g;
-                citems[2 * nc + 1] = (int32_t)p;
-                nc++;
-            }
-        }
-        r = upload(b, (void **)&b->d_citems, citems, nc * 8, "batch combine items");
-        free(citems);
-        if (r != SG_OK) return r;
-        b->ncitems = (int)nc;
-    }
+    if (ni > 0) BCU(cudaMemcpy(b->d_items, b->h_items, (size_t)(ni + nc) * 8, cudaMemcpyHostToDevice), "upload items");
+    b->d_citems = b->d_items + 2 * ni;
+    b->ncitems = (int)nc;
     for (g = 0; g <= b->ng; g++) b->eval_pt_off[g] = pt_off[g];
     b->eval_coords = coords;
     b->eval_out = out;

@@ -30,7 +30,8 @@ def fake(tmp_path_factory):
     empty = out / "empty.c"
     empty.write_text("".join(f"int {n}() {{ return 0; }}\n" for n in sorted(wanted)))
     lib = str(out / "libfake.so")
-    subprocess.run(cc + ["-shared", str(empty)] + objs + ["-o", lib, "-lpthread"], check=True)
+    # -Bsymbolic: its own CUDA runtime, whatever else the process has loaded
+    subprocess.run(cc + ["-shared", "-Wl,-Bsymbolic", str(empty)] + objs + ["-o", lib, "-lpthread"], check=True)
     so = C.CDLL(lib)
     for name, (res, args) in _lib.SIGNATURES.items():
         if hasattr(so, name):
@@ -163,3 +164,31 @@ def test_timings_are_of_the_latest_call(fake):
         assert fake.sg_timings(g.h, ms.ctypes.data) == _lib.SG_OK
         assert (ms[1] >= 0) == ordered and ms[2] >= 0, m
     g.close()
+
+
+def test_batch_plans_reuse_their_memory(fake):
+    """New offsets or buffers make a new plan; beyond the points' own ordering
+    buffers it allocates only what it has no room for."""
+    dims, levels = np.array([6, 8, 10], np.int32), np.array([9, 7, 7], np.int32)
+    start = fake.fake_live()
+    b = C.c_void_p()
+    assert fake.sg_batch_create(3, dims.ctypes.data, levels.ctypes.data, None, C.byref(b)) == _lib.SG_OK
+    off = np.zeros(4, np.int64)
+    fake.sg_batch_offsets(b, off.ctypes.data)
+    values = np.zeros(off[3], np.float32)
+    assert fake.sg_batch_set_values(b, values.ctypes.data) == _lib.SG_OK
+    assert fake.sg_batch_set_option(b, _lib.SG_OPT_EVAL_SORT, 0) == _lib.SG_OK
+    x = np.zeros(10 * 4000, np.float32)
+
+    def evaluate(counts):
+        po = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+        before = fake.fake_allocs(), fake.fake_frees()
+        assert fake.sg_batch_evaluate_device(b, po.ctypes.data, x.ctypes.data, x.ctypes.data, None) == _lib.SG_OK
+        return fake.fake_allocs() - before[0], fake.fake_frees() - before[1]
+
+    evaluate([1000, 900, 800])
+    for counts in ([999, 901, 800], [1, 0, 700], [1000, 900, 800]):
+        assert evaluate(counts) == (0, 0), counts
+    assert evaluate([1500, 1000, 800])[0] > 0
+    assert fake.sg_batch_destroy(b) == _lib.SG_OK
+    assert fake.fake_live() == start
