@@ -431,14 +431,23 @@ int sg_layout_pass(const sg_layout *L, int k0, int g, sg_pass_host *p)
 
 int64_t sg_layout_sweep_bytes(const sg_layout *L)
 {
-    int64_t b = 0;
-    int k, g;
+    int64_t bytes = 0;
+    int k, g, s, a, b, c;
     for (k = 0; k < L->d; k += g > 0 ? g : 1) {
         g = sg_layout_pass_dims(L, k, 4);
-        if (g > 0) b += (8 * g + 2) * pass_nodes(L, k, g, L->n - 1) + 8 * SG_MAX_LEVELS * SG_MAX_LEVELS * SG_MAX_LEVELS / 8;
-        b += 12 * L->S + 4096; /* chains or units, and subspace offsets */
+        /* chains or units of two subspaces at least (8 bytes each), and an
+         * offset per subspace */
+        bytes += 8 * L->S;
+        if (!g) continue;
+        bytes += (int64_t)(g * sizeof(sg_unit_node) + 2) * pass_nodes(L, k, g, L->n - 1);
+        for (s = 0; s < L->n; s++)
+            for (a = 0; a <= s && a <= L->lim[k]; a++)
+                for (b = 0; a + b <= s && b <= (g > 1 ? L->lim[k + 1] : 0); b++) {
+                    c = s - a - b;
+                    if (c <= (g > 2 ? L->lim[k + 2] : 0)) bytes += sizeof(sg_unit_combo);
+                }
     }
-    return b;
+    return bytes;
 }
 
 /* ---- evaluation (block) layout ------------------------------------------ */
