@@ -39,9 +39,9 @@
  *   - most blocks sit under walk nodes of small remaining budget (at d=10,
  *     n=10, 8,008 of 11,440 blocks hold at most 4 subspaces), where loop and
  *     dispatch cost more than the gathers: the last prefix dim with budget
- *     <= SG_EVAL_MAX_LEAF (levels and blocks) and the last two with budget
- *     <= kLG2 run as fully unrolled code with compile-time block sizes, in
- *     walk order, so results are bit-identical to the loop (d <= kMaxUnrollD);
+ *     <= kLeaf (levels and blocks) and the last two with budget <= kLeaf2 run
+ *     as fully unrolled code with compile-time block sizes, in walk order, so
+ *     results are bit-identical to the loop;
  *   - per prefix dim the walk keeps three values per point: the fractional
  *     part y = frac(x 2^l) (next level: doubling, exact in FP32), the cell
  *     index of the prefix (next level: 2*ix + bit) and the parent's product;
@@ -551,15 +551,19 @@ __device__ __noinline__ uint32_t close_segment(Tail<P> *t, FV<P> v)
     return s + 2 < t->nseg ? __ldg(t->bounds + s + 2) : 0xFFFFFFFFu;
 }
 
-/* largest budget of an unrolled leaf subtree of the last two prefix dims (of
- * the last one: SG_EVAL_MAX_LEAF) */
-constexpr int kLG2 = SG_EVAL_MAX_LEAF2;
-static_assert(kLG2 == SG_SEG_UNIT_BUDGET, "segments start outside the unrolled subtrees");
-static_assert(SG_EVAL_MAX_LEAF <= 5 && kLG2 <= 3,
+/* Largest budgets of the unrolled subtrees of the last prefix dim (kLeaf) and of
+ * the last two (kLeaf2).  Above 12 dims the walk's own loops take most of the
+ * time and the small subtrees most of the gain, while the unrolled code takes
+ * ptxas four to ten times as long with the budgets of the lower dims.  Whole sums
+ * with loops only / these budgets / 5 and 3: d = 13, n = 6, 5e5 points 7.43 /
+ * 4.39 / 3.99 ms, d = 16, n = 5, 3e5 points 3.17 / 2.18 / 2.34 ms. */
+template <int D>
+constexpr int kLeaf = D <= 12 ? SG_EVAL_MAX_LEAF : 2;
+template <int D>
+constexpr int kLeaf2 = D <= 12 ? SG_EVAL_MAX_LEAF2 : 1;
+static_assert(SG_EVAL_MAX_LEAF2 == SG_SEG_UNIT_BUDGET, "segments start outside the unrolled subtrees");
+static_assert(SG_EVAL_MAX_LEAF <= 5 && SG_EVAL_MAX_LEAF2 <= 3,
               "the walk's jump tables cover leaf budgets 0..5 and 0..3");
-/* unrolled subtrees are instantiated for d <= kMaxUnrollD only (their code
- * grows with d; grids of more dims keep the loop) */
-constexpr int kMaxUnrollD = 12;
 
 /* next level of one prefix dim for every point: y doubles, the cell index
  * takes the next bit */
@@ -720,30 +724,36 @@ struct Walk {
         uint32_t ix[P];
 #pragma unroll
         for (int p = 0; p < P; ++p) ix[p] = ixin[p];
-        if constexpr (D <= kMaxUnrollD && K + 1 == D - 4) {
-            if (budget <= kLG2 && budget <= A.lim[K] && budget <= A.lim[K + 1] && budget <= A.lim3) {
+        if constexpr (K + 1 == D - 4) {
+            if (budget <= kLeaf2<D> && budget <= A.lim[K] && budget <= A.lim[K + 1] && budget <= A.lim3) {
                 switch (budget) {
                 case 0: leaf_group2<D, K, P, 0, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
                 case 1: leaf_group2<D, K, P, 1, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
-                case 2: leaf_group2<D, K, P, 2, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
-                case 3: leaf_group2<D, K, P, 3, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp); break;
+                case 2:
+                    if constexpr (kLeaf2<D> >= 2) leaf_group2<D, K, P, 2, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp);
+                    break;
+                case 3:
+                    if constexpr (kLeaf2<D> >= 3) leaf_group2<D, K, P, 3, 0>(A, sx, tid, cur, in, pin, y, ix, sum, comp);
+                    break;
                 default: break;
                 }
                 return;
             }
         }
-        if constexpr (D <= kMaxUnrollD && K == D - 4) {
-            if (budget <= SG_EVAL_MAX_LEAF && budget <= A.lim[K] && budget <= A.lim3) {
+        if constexpr (K == D - 4) {
+            if (budget <= kLeaf<D> && budget <= A.lim[K] && budget <= A.lim3) {
                 switch (budget) {
                 case 0: leaf_group<D, P, 0, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 1: leaf_group<D, P, 1, 0>(A, cur, in, pin, y, ix, acc); break;
                 case 2: leaf_group<D, P, 2, 0>(A, cur, in, pin, y, ix, acc); break;
-                case 3: leaf_group<D, P, 3, 0>(A, cur, in, pin, y, ix, acc); break;
+                case 3:
+                    if constexpr (kLeaf<D> >= 3) leaf_group<D, P, 3, 0>(A, cur, in, pin, y, ix, acc);
+                    break;
                 case 4:
-                    if constexpr (SG_EVAL_MAX_LEAF >= 4) leaf_group<D, P, 4, 0>(A, cur, in, pin, y, ix, acc);
+                    if constexpr (kLeaf<D> >= 4) leaf_group<D, P, 4, 0>(A, cur, in, pin, y, ix, acc);
                     break;
                 case 5:
-                    if constexpr (SG_EVAL_MAX_LEAF >= 5) leaf_group<D, P, 5, 0>(A, cur, in, pin, y, ix, acc);
+                    if constexpr (kLeaf<D> >= 5) leaf_group<D, P, 5, 0>(A, cur, in, pin, y, ix, acc);
                     break;
                 default: break;
                 }
