@@ -863,6 +863,8 @@ static int tune_hier_once(sg_grid *g, void *a)
     return hierarchize_on(g, t->st);
 }
 
+static int plan_sort(const sg_grid *g, int64_t m);
+
 SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_evals, void *stream, double *ms)
 {
     static const int ppts[2] = {1, 2};
@@ -892,7 +894,9 @@ SG_API int sg_autotune(sg_grid *g, const float *coords, float *out, int64_t num_
         }
     if (r == SG_OK) {
         g->opt[SG_OPT_EVAL_PPT] = ppts[bi / 2];
-        g->opt[SG_OPT_EVAL_SORT] = bi % 2;
+        /* ordering that is not done at this size was not timed either */
+        g->opt[SG_OPT_EVAL_SORT] = 1;
+        g->opt[SG_OPT_EVAL_SORT] = plan_sort(g, num_evals) ? bi % 2 : opt[SG_OPT_EVAL_SORT];
     }
     /* under each blocking value (one kernel form: two timings of the same) */
     for (i = 0, best = 1e30, bi = -1; i < SG_EVAL_BLOCKINGS && r == SG_OK; i++) {

@@ -64,7 +64,8 @@ extern "C" {
 #define SG_OPT_EVAL_PPT 3       /* 0, 1 or 2, without effect: every thread takes two */
                                 /* points, and few points share their sums among     */
                                 /* warps                                             */
-#define SG_OPT_HIER_KERNEL 5    /* 0 = auto, 1 = shared-memory chains, 2 = gather,   */
+#define SG_OPT_HIER_KERNEL 5    /* 0 = auto, 1 = staged in shared memory (passes of  */
+                                /* several dims, and single-dim chains), 2 = gather, */
                                 /* 3 = one warp per chain (batches only)            */
 #define SG_OPT_PROFILE 6        /* 1: record CUDA events around each phase            */
 #define SG_OPT_USE_GRAPH 7      /* batches: 1 (default) capture launches in a CUDA graph */
@@ -164,10 +165,11 @@ int sg_sync(sg_grid *grid, void *stream);
  * the evaluation under every setting of SG_OPT_EVAL_PPT {1, 2} x spatial
  * ordering {off, on}, then, at the faster of those, under every value of
  * SG_OPT_EVAL_BLOCKING (1..2), and the hierarchization with the
- * shared-memory chain sweeps (where they fit) and the gather sweeps; keeps
+ * shared-memory sweeps (where they fit) and the gather sweeps; keeps
  * the fastest in the handle's options (SG_OPT_EVAL_PPT, SG_OPT_EVAL_SORT,
- * SG_OPT_EVAL_BLOCKING, SG_OPT_HIER_KERNEL).  No setting changes any result.
- * The grid's values are the same on return (saved and restored); out[] holds
+ * SG_OPT_EVAL_BLOCKING, SG_OPT_HIER_KERNEL); SG_OPT_EVAL_SORT stays as it was
+ * where so many points would not be ordered anyway.  No setting changes any
+ * result.  The grid's values are the same on return (saved and restored); out[] holds
  * the evaluation.  ms (optional, SG_TUNE_TIMINGS entries): evaluation ms for
  * (ppt, sort) = (1,0), (1,1), (2,0), (2,1), then hierarchization ms for
  * chains and gather, then evaluation ms for blocking 1, 2 (-1: not

@@ -192,3 +192,17 @@ def test_batch_plans_reuse_their_memory(fake):
     assert evaluate([1500, 1000, 800])[0] > 0
     assert fake.sg_batch_destroy(b) == _lib.SG_OK
     assert fake.fake_live() == start
+
+
+@pytest.mark.parametrize("sort", [0, 1])
+def test_autotune_leaves_an_untimed_setting_alone(fake, sort):
+    """Few points are not ordered under either setting, so the tuner has nothing
+    to choose from (all timings are equal here) and a later call with many points
+    finds the setting that the caller made."""
+    g = Grid(fake, 6, 9)
+    assert g.set_values() == _lib.SG_OK
+    assert fake.sg_set_option(g.h, _lib.SG_OPT_EVAL_SORT, sort) == _lib.SG_OK
+    x, ms, v = np.zeros(600, np.float32), np.zeros(_lib.SG_TUNE_TIMINGS), C.c_int64()
+    assert fake.sg_autotune(g.h, x.ctypes.data, x.ctypes.data, 100, None, ms.ctypes.data) == _lib.SG_OK
+    assert fake.sg_get_option(g.h, _lib.SG_OPT_EVAL_SORT, C.byref(v)) == _lib.SG_OK and v.value == sort
+    g.close()
