@@ -323,6 +323,14 @@ def repo_libraries() -> list:
     return sorted(libs)
 
 
+def reference_missing():
+    """Why the reference's CPU code cannot run here, None where it can."""
+    from oracle.oracle import Reference
+    if Reference.available():
+        return None
+    return "oracle/_ref/libasgb_ref.so is not built: the reference's sources are not on this machine"
+
+
 def run_reference_arm(args, rank: int, world: int):
     """The reference's CPU implementation (oracle/_ref) on the default
     workload; inputs come from the checker side (oracle/) only, so the
@@ -336,6 +344,9 @@ def run_reference_arm(args, rank: int, world: int):
                 "unavailable": "the reference arm times the default single-grid workload only"}
     from oracle import workload as owl
     from oracle.oracle import Oracle
+    missing = reference_missing()
+    if missing:
+        return {"impl": "reference", "unavailable": missing}
     vals = owl.grid_values(Oracle(D, NLEV), owl.f_gauss)
     m_step = args.points or M_EVAL
     X = owl.uniform_points(SEED, min(m_step, 1 << 20), D)
@@ -577,7 +588,10 @@ def run_b200(args, rank: int, world: int, local_rank: int, wl=None, extras: bool
         "autotune_ms": tuned,
         "clocks": clocks,
     }
-    if world == 1 and not args.no_cpu_baseline:
+    if world == 1 and not args.no_cpu_baseline and reference_missing():
+        line["cpu_baseline"] = {"unavailable": reference_missing()}
+        line["err_vs_fp64"] = error_vs_fp64(vals_d.cpu().numpy(), out_d.cpu().numpy(), X, wl=wl)
+    elif world == 1 and not args.no_cpu_baseline:
         vals = vals_d.cpu().numpy()
         cpu_v, info = reference_cpu(vals, X[:1 << 20], cpu_step_seconds(args), wl,
                                     one_thread_points=4096 if extras else 0)
