@@ -496,8 +496,11 @@ struct Tail {
     bool valid[P], nan_in[P];
 };
 
+/* adds the compensated sum (vs, vc) to acc, its compensation included: a segment
+ * rounded to one float where it ends would cost up to 5 % in the error of the
+ * total */
 template <int P>
-__device__ __forceinline__ void fold(float (&acc)[2][P], FV<P> v)
+__device__ __forceinline__ void fold(float (&acc)[2][P], FV<P> vs, FV<P> vc)
 {
     FV<P> s, c;
 #pragma unroll
@@ -505,7 +508,8 @@ __device__ __forceinline__ void fold(float (&acc)[2][P], FV<P> v)
         s.set(p, acc[0][p]);
         c.set(p, acc[1][p]);
     }
-    kahan_add(s, c, v);
+    kahan_add(s, c, vs);
+    kahan_add(s, c, vsub(FV<P>::all(0.0f), vc));
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         acc[0][p] = s.get(p);
@@ -513,40 +517,43 @@ __device__ __forceinline__ void fold(float (&acc)[2][P], FV<P> v)
     }
 }
 
+/* moves the compensated sum in acc out */
 template <int P>
-__device__ __forceinline__ FV<P> take(float (&acc)[2][P])
+__device__ __forceinline__ void take(float (&acc)[2][P], FV<P> &s, FV<P> &c)
 {
-    FV<P> s, c;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         s.set(p, acc[0][p]);
         c.set(p, acc[1][p]);
         acc[0][p] = acc[1][p] = 0.0f;
     }
-    return vsub(s, c);
 }
 
-/* Ends the current segment, whose sum is v; returns the next segment's end. */
+/* Ends the current segment, whose compensated sum is (v, c); returns the next
+ * segment's end. */
 template <int P>
-__device__ __noinline__ uint32_t close_segment(Tail<P> *t, FV<P> v)
+__device__ __noinline__ uint32_t close_segment(Tail<P> *t, FV<P> v, FV<P> c)
 {
     const int s = t->s++;
     int k = s;
     bool whole = true;
     if (t->emit != SG_EMIT_SEGS) {
-        fold<P>(t->part, v);
+        fold<P>(t->part, v, c);
         whole = (s + 1) % SG_SEG_PER_PART == 0 || s + 1 == t->nseg;
         if (whole) {
-            v = take<P>(t->part);
+            take<P>(t->part, v, c);
             k = s / SG_SEG_PER_PART;
-            if (t->emit == SG_EMIT_SUM) fold<P>(t->total, v);
+            if (t->emit == SG_EMIT_SUM) fold<P>(t->total, v, c);
         }
     }
     if (whole && t->emit != SG_EMIT_SUM) {
 #pragma unroll
         for (int p = 0; p < P; ++p)
-            if (t->out[p])
-                t->out[p][k * t->stride] = t->valid[p] ? v.get(p) : (t->nan_in[p] ? __int_as_float(0x7fc00000) : 0.0f);
+            if (t->out[p]) {
+                t->out[p][2 * k * t->stride] =
+                    t->valid[p] ? v.get(p) : (t->nan_in[p] ? __int_as_float(0x7fc00000) : 0.0f);
+                t->out[p][(2 * k + 1) * t->stride] = t->valid[p] ? c.get(p) : 0.0f;
+            }
     }
     return s + 2 < t->nseg ? __ldg(t->bounds + s + 2) : 0xFFFFFFFFu;
 }
@@ -658,7 +665,7 @@ struct Walk {
     static __device__ __forceinline__ bool close(Range &rg, Tail<P> *tl, uint32_t cur, FV<P> &sum, FV<P> &comp)
     {
         while (cur >= rg.next) {
-            rg.next = close_segment<P>(tl, vsub(sum, comp));
+            rg.next = close_segment<P>(tl, sum, comp);
             sum = comp = FV<P>::all(0.0f);
             if constexpr (SH) {
                 if (tl->s >= tl->end) {
@@ -910,12 +917,11 @@ __device__ __forceinline__ void eval_points(const EvalArgs &A, const GA &G, floa
         Walk<D, 0, P, SH>::run(G, sx, tid, A.nm1, cur, rg, &tl, in, xC, xA, xB, pin, ix, sum, comp);
         if (A.nseg > 1) {
             while (tl.s < tl.end) {
-                (void)close_segment<P>(&tl, vsub(sum, comp));
+                (void)close_segment<P>(&tl, sum, comp);
                 sum = comp = FV<P>::all(0.0f);
             }
             if (A.emit != SG_EMIT_SUM) return;
-            sum = take<P>(tl.total);
-            comp = FV<P>::all(0.0f);
+            take<P>(tl.total, sum, comp);
         }
     } else {
         uint32_t base[P];

@@ -32,8 +32,9 @@ __device__ __forceinline__ void kahan(float &s, float &c, float v)
     s = t;
 }
 
-/* Total of one point from what its warps wrote: the parts, or the segments
- * part by part, in order and compensated as eval_impl.cuh adds them. */
+/* Total of one point from the compensated sums that its warps wrote (sum, then
+ * compensation): the parts, or the segments part by part, in the order and
+ * arithmetic of eval_impl.cuh. */
 __device__ __forceinline__ float combine(const float *__restrict__ src, int64_t m, int nseg, int nparts, int emit)
 {
     float s = 0.0f, c = 0.0f;
@@ -41,18 +42,25 @@ __device__ __forceinline__ float combine(const float *__restrict__ src, int64_t 
      * arithmetic one */
     if (__float_as_uint(src[0]) == 0x7fc00000u) return src[0];
     if (emit == SG_EMIT_PARTS) {
-        for (int k = 0; k < nparts; ++k) kahan(s, c, src[k * m]);
+        for (int k = 0; k < nparts; ++k) {
+            kahan(s, c, src[2 * k * m]);
+            kahan(s, c, __fsub_rn(0.0f, src[(2 * k + 1) * m]));
+        }
         return __fsub_rn(s, c);
     }
     for (int k0 = 0; k0 < nseg; k0 += SG_SEG_PER_PART) {
         float ps = 0.0f, pc = 0.0f;
-        float v[SG_SEG_PER_PART];
+        float v[2 * SG_SEG_PER_PART];
 #pragma unroll
-        for (int k = 0; k < SG_SEG_PER_PART; ++k) v[k] = k0 + k < nseg ? src[(k0 + k) * m] : 0.0f;
+        for (int k = 0; k < 2 * SG_SEG_PER_PART; ++k) v[k] = k0 + k / 2 < nseg ? src[(2 * k0 + k) * m] : 0.0f;
 #pragma unroll
         for (int k = 0; k < SG_SEG_PER_PART; ++k)
-            if (k0 + k < nseg) kahan(ps, pc, v[k]);
-        kahan(s, c, __fsub_rn(ps, pc));
+            if (k0 + k < nseg) {
+                kahan(ps, pc, v[2 * k]);
+                kahan(ps, pc, __fsub_rn(0.0f, v[2 * k + 1]));
+            }
+        kahan(s, c, ps);
+        kahan(s, c, __fsub_rn(0.0f, pc));
     }
     return __fsub_rn(s, c);
 }

@@ -95,8 +95,9 @@ typedef struct sg_eval_plan {
 #define SG_EVAL_MAX_PARTS 8
 
 /* What a launch writes of a point's sum: all of it to out; or, when several
- * warps share it, each its parts or segments to part_out (value k of point i
- * at part_out[k * num_evals + i]), added afterwards by sgk_combine_*. */
+ * warps share it, each its parts or segments to part_out (sum k of point i at
+ * part_out[2 k * num_evals + i], its compensation at part_out[(2 k + 1) *
+ * num_evals + i]), added afterwards by sgk_combine_*. */
 #define SG_EMIT_SUM 0
 #define SG_EMIT_PARTS 1
 #define SG_EMIT_SEGS 2

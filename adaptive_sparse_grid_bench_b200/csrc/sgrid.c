@@ -1008,8 +1008,9 @@ static void grid_plan(const sg_grid *g, sg_eval_plan *p)
  * per SM, 64 points each) the segments of a sum go to several warps.  (The
  * kernel that can share is about a quarter slower per point than the one that
  * cannot; above 12 dims, where its walk down to each segment is long, twice as
- * slow, so there only below a quarter: d = 16, n = 5, 65,536 points 1.2 ms whole and
- * 2.1 ms shared before the small subtrees were unrolled there; 0.89 ms whole since.)  d = 10, n = 10: 7.35 -> 0.17 ms for 1,000 points, 6.05 -> 3.3 ms for
+ * slow, so there only below a quarter: d = 16, n = 5, 65,536 points 1.2 ms whole
+ * and 2.1 ms shared before the small subtrees were unrolled there, 0.89 ms whole
+ * since.)  d = 10, n = 10: 7.35 -> 0.17 ms for 1,000 points, 6.05 -> 3.3 ms for
  * 65,536; 2^20 points share at a loss (35.3 -> 42.9 ms).  Returns the floats of
  * part_out (0: whole sums).  No choice changes a result. */
 static int64_t plan_shares(const sg_grid *g, int64_t m, sg_eval_plan *p)
@@ -1023,11 +1024,11 @@ static int64_t plan_shares(const sg_grid *g, int64_t m, sg_eval_plan *p)
     if (want <= p->nparts) {
         p->nshare = p->nparts;
         p->emit = SG_EMIT_PARTS;
-        floats = p->nparts * m;
+        floats = 2 * p->nparts * m;
     } else {
         p->nshare = want < p->nseg ? (int)want : p->nseg;
         p->emit = SG_EMIT_SEGS;
-        floats = p->nseg * m;
+        floats = 2 * p->nseg * m;
     }
     if (floats <= SG_SHARE_FLOATS) return floats;
     p->nshare = 1;

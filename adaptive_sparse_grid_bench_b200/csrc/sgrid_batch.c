@@ -969,7 +969,7 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
         cap_items += (m + SG_EVAL_CTA_POINTS - 1) / SG_EVAL_CTA_POINTS * ns;
         if (ns > 1) {
             cap_c += (m + 255) / 256;
-            parts += m * (sg_layout_parts(&b->L[g]) > 1 ? sg_layout_parts(&b->L[g]) : sg_layout_segs(&b->L[g]));
+            parts += 2 * m * (sg_layout_parts(&b->L[g]) > 1 ? sg_layout_parts(&b->L[g]) : sg_layout_segs(&b->L[g]));
         }
     }
     if (parts > b->part_floats) {
@@ -1021,7 +1021,7 @@ static int plan_eval(sg_batch *b, const int64_t *pt_off, const float *coords, fl
         p.nshare = batch_shares(L, ctas);
         p.emit = p.nshare > 1 ? (p.nparts > 1 ? SG_EMIT_PARTS : SG_EMIT_SEGS) : SG_EMIT_SUM;
         p.part_out = b->d_part + parts;
-        if (p.nshare > 1) parts += (pt_off[g + 1] - pt_off[g]) * (p.nparts > 1 ? p.nparts : p.nseg);
+        if (p.nshare > 1) parts += 2 * (pt_off[g + 1] - pt_off[g]) * (p.nparts > 1 ? p.nparts : p.nseg);
         sgk_fill_eval_args(&p, coords + coff, NULL, out + pt_off[g], pt_off[g + 1] - pt_off[g], &b->h_eval_args[g]);
         coff += (pt_off[g + 1] - pt_off[g]) * L->d;
     }

@@ -372,7 +372,7 @@ static int take_batch(sg_server *s, srv_slot *sl)
         sl->out_off[sl->nreq] = pts;
         sl->coord_off[sl->nreq] = coff;
         sl->part_off[sl->nreq] = poff;
-        if (sg_layout_parts(&r->g->L) > 1 && !whole_sums(r)) poff += r->m * sg_layout_parts(&r->g->L);
+        if (sg_layout_parts(&r->g->L) > 1 && !whole_sums(r)) poff += 2 * r->m * sg_layout_parts(&r->g->L);
         coff += r->m * r->d;
         pts += r->m;
         sl->nreq++;
@@ -664,7 +664,7 @@ SG_API int sg_server_create(int64_t hbm_cap_bytes, int64_t max_batch_points, sg_
             cudaMallocHost((void **)&sl->h_items, (size_t)max_items * 8) != cudaSuccess ||
             cudaMallocHost((void **)&sl->h_citems, (size_t)max_items * 8) != cudaSuccess ||
             cudaMalloc((void **)&sl->d_citems, (size_t)max_items * 8) != cudaSuccess ||
-            cudaMalloc((void **)&sl->d_part, ob * SG_EVAL_MAX_PARTS) != cudaSuccess ||
+            cudaMalloc((void **)&sl->d_part, 2 * ob * SG_EVAL_MAX_PARTS) != cudaSuccess ||
             cudaMalloc((void **)&sl->d_coords, cb) != cudaSuccess || cudaMalloc((void **)&sl->d_out, ob) != cudaSuccess ||
             cudaMalloc((void **)&sl->d_args, SRV_MAX_REQS * sizeof(sg_eval_args)) != cudaSuccess ||
             cudaMalloc((void **)&sl->d_items, (size_t)max_items * 8) != cudaSuccess ||

@@ -75,3 +75,25 @@ def test_a_non_finite_surplus_stays_in_its_cell(cuda, d, n, level, value):
     assert inside.sum() >= 500 and away.sum() > 100
     assert not np.any(np.isfinite(out[inside]))
     assert np.array_equal(out[away].view(np.uint32), clean[away].view(np.uint32))
+
+
+def test_segments_keep_their_compensation(cuda):
+    """2^24 + 1 inside one segment and -2^24 in another: the 1, which no float
+    beside 2^24 holds, survives the segment's end, in whole and in shared sums."""
+    import torch
+    d, n = 10, 7
+    g = sg.Grid(d, n)
+    s = np.zeros(g.num_points, np.float32)
+    # at x = 1/4 the hats are 1/2 at level 0, 1 at level 1 and 0 above; the first
+    # two are neighbours in the walk, in a subtree that no segment divides
+    for levels, value in (((1, 1, 1, 0, 0, 0, 0, 0, 0, 0), 2.0 ** 24), ((1, 1, 1, 0, 0, 1, 0, 0, 0, 0), 1.0),
+                          ((0,) * 10, -2.0 ** 24)):
+        s[g.gp2idx(levels, (0,) * d)] = value * 2.0 ** (d - sum(levels))
+    g.set_values(s)
+    m = torch.cuda.get_device_properties(cuda).multi_processor_count * 16 * 64
+    X = torch.full((m, d), 0.25, device=cuda)
+    for k in (1, 1000, m):
+        out = torch.empty(k, device=cuda)
+        g.evaluate_device(X, out, k)
+        g.sync()
+        assert bool((out == 1.0).all()), (k, float(out[0]))
