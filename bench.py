@@ -57,10 +57,10 @@ EVAL_SRC = os.path.join(ROOT, "adaptive_sparse_grid_bench_b200", "csrc", "eval_i
 #   dram_bytes: dram__bytes_read.sum + dram__bytes_write.sum of one full
 #     2^24-point launch (one-pass metrics, so the full launch was captured);
 #   inst_per_pair: smsp__inst_executed.sum x 32 / (points x subspaces) of a
-#     1,048,576-point launch of the same grid (two points per thread, wide preset).
+#     1,048,576-point launch of the same grid.
 #   (either may be None: not captured on this source)
-EVAL_CAPTURE = {"source_sha16": "ab15c4c8da0625a8", "captured": "2026-12-04", "dram_bytes": 2.953e9 + 0.588e9,
-                "inst_per_pair": 7.14}
+EVAL_CAPTURE = {"source_sha16": "ff45ae5461536e37", "captured": "2026-12-05", "dram_bytes": 2.852e9 + 0.789e9,
+                "inst_per_pair": 6.56}
 SM_COUNT, SCHEDULERS_PER_SM = 148, 4
 
 
