@@ -109,7 +109,7 @@ def test_captured_evaluations_share_their_sums(cuda):
     torch.cuda.synchronize()
     for o, w in zip(got, want):
         assert torch.equal(_bits(o), _bits(w))
-    # 128 segments x 10,000 points x 4 bytes: room for 24 more beside these two
+    # 128 segments x 10,000 points x 8 bytes: room for 12 more beside these two
     launches = []
     for _ in range(30):
         graph = torch.cuda.CUDAGraph()

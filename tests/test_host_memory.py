@@ -206,3 +206,35 @@ def test_autotune_leaves_an_untimed_setting_alone(fake, sort):
     assert fake.sg_autotune(g.h, x.ctypes.data, x.ctypes.data, 100, None, ms.ctypes.data) == _lib.SG_OK
     assert fake.sg_get_option(g.h, _lib.SG_OPT_EVAL_SORT, C.byref(v)) == _lib.SG_OK and v.value == sort
     g.close()
+
+
+def test_memory_of_shared_sums(fake):
+    """A call that shares its sums returns their memory with its last launch, does
+    without where there is none, and allocates under capture only what the handle
+    keeps."""
+    start = fake.fake_live()
+    g = Grid(fake, 6, 9)
+    assert g.set_values() == _lib.SG_OK
+    x = np.zeros((100, 6), np.float32)
+
+    def evaluate(stream=None):
+        return fake.sg_evaluate_device(g.h, x.ctypes.data, x.ctypes.data, 100, stream)
+
+    assert evaluate() == _lib.SG_OK and fake.fake_pool_live() == 0
+    live, allocs = fake.fake_live(), fake.fake_allocs()
+    assert evaluate() == _lib.SG_OK and (fake.fake_live(), fake.fake_allocs()) == (live, allocs + 1)
+    fake.fake_fail(0)
+    assert evaluate() == _lib.SG_OK and fake.fake_pool_live() == 0
+    unsafe = fake.fake_unsafe()
+    fake.fake_capture(12345)
+    try:
+        assert evaluate(12345) == _lib.SG_OK and fake.fake_live() == live + 1
+        assert evaluate() == _lib.SG_OK  # beside the capture
+        fake.fake_fail(0)
+        assert evaluate(12345) == _lib.SG_OK and fake.fake_live() == live + 1
+    finally:
+        fake.fake_capture(None)
+        fake.fake_fail(-1)
+    assert fake.fake_unsafe() == unsafe and fake.fake_pool_live() == 0
+    g.close()
+    assert fake.fake_live() == start
